@@ -250,12 +250,11 @@ __device__ __forceinline__ void matvec_epilogue(const MatvecArgs& a, const float
   }
 }
 
-// NW warps of RW rows (dual: of both matrices) each.
-template <int WT, int B, bool DUAL, int RW, int NW>
-__global__ void __launch_bounds__(32 * NW, NW == 16 ? 2 : 0) matvec_q_kernel(const MatvecArgs a) {
+template <int WT, int B, bool DUAL, int RW>
+__global__ void __launch_bounds__(256) matvec_q_kernel(const MatvecArgs a) {
   extern __shared__ __align__(16) uint8_t smem[];
-  constexpr int R = NW * RW;   // rows per CTA
-  static_assert(!DUAL || R == 32, "the SwiGLU epilogue quantizes 32-row blocks");
+  constexpr int R = 8 * RW;   // rows per CTA
+  static_assert(!DUAL || RW == 4, "the SwiGLU epilogue quantizes 32-row blocks");
   const int U = a.K / 32;
   {
     // This CTA's weight rows are one contiguous range (two when dual).  Ask for them in L2 now: the
@@ -269,7 +268,7 @@ __global__ void __launch_bounds__(32 * NW, NW == 16 ? 2 : 0) matvec_q_kernel(con
       constexpr uint32_t CH = 16384;
       const int nch = (int)((total + CH - 1) / CH);
       const uint8_t* base = a.w + (size_t)r0 * (DUAL ? 2 : 1) * rbp;
-      for (int c = threadIdx.x; c < nch; c += 32 * NW) {
+      for (int c = threadIdx.x; c < nch; c += 256) {
         const size_t off = (size_t)c * CH;
         prefetch_l2(base + off, (uint32_t)min((size_t)CH, total - off));
       }
@@ -286,7 +285,7 @@ __global__ void __launch_bounds__(32 * NW, NW == 16 ? 2 : 0) matvec_q_kernel(con
 
   // Stage the quantized activations (a few KB per token) into shared memory, split into two
   // 16-byte planes so a warp's reads are conflict-free.
-  for (int i = tid; i < B * U; i += 32 * NW) {
+  for (int i = tid; i < B * U; i += 256) {
     const int b = i / U, u = i - b * U;
     if (b < a.nb) {
       const uint4* src = (const uint4*)(a.xq + (size_t)b * a.K + (size_t)u * 32);
@@ -318,7 +317,7 @@ __global__ void __launch_bounds__(32 * NW, NW == 16 ? 2 : 0) matvec_q_kernel(con
   bool live[RW];
 #pragma unroll
   for (int i = 0; i < RW; i++) {
-    const int n = blockIdx.x * R + w + NW * i;
+    const int n = blockIdx.x * R + w + 8 * i;
     live[i] = n < a.N;
     const int nn = live[i] ? n : 0;
 #pragma unroll
@@ -329,7 +328,7 @@ __global__ void __launch_bounds__(32 * NW, NW == 16 ? 2 : 0) matvec_q_kernel(con
     }
   }
   // Load phase (all rows of the warp, both matrices) then compute phase, per 32-unit column block.
-#pragma unroll(NW == 16 ? 1 : 2)
+#pragma unroll 2
   for (int u = lane; u < U; u += 32) {
     UnitRaw<WT> raw[NM][RW];
 #pragma unroll
@@ -343,7 +342,7 @@ __global__ void __launch_bounds__(32 * NW, NW == 16 ? 2 : 0) matvec_q_kernel(con
   }
 #pragma unroll
   for (int i = 0; i < RW; i++) {
-    const int r = w + NW * i;
+    const int r = w + 8 * i;
 #pragma unroll
     for (int b = 0; b < B; b++) {
       float v0 = warp_sum(acc[0][i][b]);
@@ -443,17 +442,17 @@ __global__ void __launch_bounds__(256) matvec_bf16_kernel(const MatvecArgs a) {
   if (a.epi == EPI_ALLREDUCE) sym_kernel_end_barrier(a.sym, 0, gridDim.x, a.wait_ready != 0);
 }
 
-template <int WT, int B, bool DUAL, int RW, int NW = 8>
+template <int WT, int B, bool DUAL, int RW>
 static int launch_q_rw(const MatvecArgs& a, cudaStream_t st) {
   const int U = a.K / 32;
   const size_t smem = (size_t)B * U * (16 + 16 + 4 + 8) + 2 * 32 * B * sizeof(float);
-  auto kern = matvec_q_kernel<WT, B, DUAL, RW, NW>;
+  auto kern = matvec_q_kernel<WT, B, DUAL, RW>;
   if (smem > 48 * 1024) {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return (int)e;
   }
-  constexpr int R = NW * RW;
-  return launch_pdl(kern, dim3((a.N + R - 1) / R), dim3(32 * NW), smem, st, a);
+  constexpr int R = 8 * RW;
+  return launch_pdl(kern, dim3((a.N + R - 1) / R), dim3(256), smem, st, a);
 }
 template <int WT, int B, bool DUAL>
 static int launch_q(const MatvecArgs& a, cudaStream_t st) {
@@ -462,7 +461,6 @@ static int launch_q(const MatvecArgs& a, cudaStream_t st) {
   if constexpr (!DUAL && B <= 2) {
     if ((a.N + 31) / 32 < 3 * 148) return launch_q_rw<WT, B, DUAL, 1>(a, st);
   }
-  if constexpr (DUAL && B == 1 && WT != WT_Q6KR) return launch_q_rw<WT, B, DUAL, 2, 16>(a, st);
   return launch_q_rw<WT, B, DUAL, 4>(a, st);
 }
 template <int B, bool DUAL, int RW>
