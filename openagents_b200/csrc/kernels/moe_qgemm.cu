@@ -34,6 +34,7 @@ constexpr int kRoles = 4, kExpWarps = 8, kThreads = 32 * (kRoles + 2 * kExpWarps
 constexpr int kMaxBlocks = 1024;                     // 64-row blocks with live rows
 constexpr size_t kSmem = 1024 + kOps * kXBytes + kRaw * kRawBytes + kMaxBlocks * 8 + (2 * kRaw + 3 * kOps + 4) * 8 + 16;
 static_assert(kSmem <= 227 * 1024, "shared memory budget");
+static_assert(kRaw % 2 == 0, "a slot of the packed ring stays with one group: its parity then tells the stage (see QTraits in qgemm_tc05.cu)");
 
 struct MoeQArgs {
   const uint2* scales;       // [ceil(K / 256)][groups * N]

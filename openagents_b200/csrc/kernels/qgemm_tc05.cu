@@ -130,6 +130,12 @@ template <int WT, int QBN> struct QTraits {
   static constexpr int RAWB = WT == QW_Q4KR ? 144 : 208;
   static constexpr int RS = WT == QW_Q4KR ? (QBN == 64 ? 6 : 5) : (QBN == 64 ? 4 : 3);
   static constexpr int kAS = QBN == 64 ? 3 : 2, kXStage = 4 * QBN * 64 * 2;
+  // A group may ask for the bytes of stage g only when those of stage g - RS, in the same slot, are known to have landed: the barrier's
+  // parity says no more than that.  With an even RS the group read that stage itself; else the other group did, and what this one
+  // knows is that the MMAs of stage g - kAS - 2 have finished (its last wait for an operand slot), g - RS among them from RS = kAS + 3 on.  Below that it
+  // waits for its operand slot first, which stands for stage g - kAS.
+  static constexpr bool kSlotFirst = RS % kDqGroups != 0 && RS < kAS + 3;
+  static_assert(kDqGroups == 2 && RS >= kAS, "a stage's slots are known to be free and landed");
 };
 
 template <int WT, int QBN>
@@ -369,6 +375,11 @@ __global__ void __launch_bounds__(kQThreads, 1) qgemm_kernel(const __grid_consta
           if (n < a.N && sb + 2 < sb1) d6_next = __half2float(a.w2[(size_t)n * nsb_total + rot_sb(sb0, sb1, sb + 2 - sb0)]);
         }
         const uint32_t rs = g % RS, s = g % kAS;
+        if constexpr (QTraits<WT, QBN>::kSlotFirst) {
+          ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(done + s), ((g / kAS) & 1) ^ 1, abort_flag));
+          if (!ok) break;
+          tc_fence_after();
+        }
         ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(raw_full + rs), (g / RS) & 1, abort_flag));
         if (!ok) break;
         const uint8_t* rowp = sR + rs * RAW_BYTES + row * RAWB;
@@ -418,9 +429,11 @@ __global__ void __launch_bounds__(kQThreads, 1) qgemm_kernel(const __grid_consta
             }
           }
           if (u == 0) {      // the first values are in registers: only now does this warp need the operand slot
-            ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(done + s), ((g / kAS) & 1) ^ 1, abort_flag));
-            if (!ok) break;
-            tc_fence_after();
+            if constexpr (!QTraits<WT, QBN>::kSlotFirst) {
+              ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(done + s), ((g / kAS) & 1) ^ 1, abort_flag));
+              if (!ok) break;
+              tc_fence_after();
+            }
           } else {           // everything this warp needs from the raw stage has been read
             __syncwarp();
             if (lane == 0) mbar_arrive(smem_u32(raw_empty + rs));
