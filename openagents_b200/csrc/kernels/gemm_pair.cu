@@ -478,6 +478,7 @@ bool pair_takes(const PairGemm& g) {
   if (g.out_16 && ((g.ldc % 8) || ((uintptr_t)g.out_16 & 15))) return false;
   if (((uintptr_t)g.bias & 15) || ((uintptr_t)g.resid_bf16 & 15) || (g.resid_bf16 && (!g.out_16 || g.N % 8))) return false;
   if (g.swiglu && (!g.out_16 || g.half_out || g.bias || g.resid_bf16 || g.act || (g.N % 32))) return false;
+  if (g.add && !g.out_f32) return false;         // 16-bit results are stored: a split would leave its share alone
   if (g.splits > 1 && (!g.add || g.act)) return false;
   if (g.groups && (g.mn_major || (!g.swiglu && !g.combine) || g.group_rows % BM)) return false;
   return true;

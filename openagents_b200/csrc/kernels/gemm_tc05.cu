@@ -788,7 +788,7 @@ B200_API int b200_gemm_bf16(const void* A, const void* B, int M, int N, int K, i
     if (tile_n == 0 && split_k == 0 && !resid_f32) {
       PairGemm g = {};
       g.A = A; g.B = B; g.M = M; g.N = N; g.K = K; g.lda = lda; g.ldb = ldb; g.mn_major = true; g.out_f32 = out_f32; g.out_16 = out_bf16;
-      g.ldc = ldc; g.bias = bias; g.resid_bf16 = resid_bf16; g.add = accumulate; g.alpha = 1.f; g.act = act; g.status = status;
+      g.ldc = ldc; g.bias = bias; g.resid_bf16 = resid_bf16; g.add = accumulate && out_f32; g.alpha = 1.f; g.act = act; g.status = status;
       if (choose_pair(g, N >= 256 && t256 >= 148 ? 256 : 128, 1)) return launch_gemm_pair(g, st);
     }
     if ((tile_n == 256 || (tile_n == 0 && N >= 256 && t256 >= 148)))
@@ -839,7 +839,7 @@ B200_API int b200_gemm_bf16(const void* A, const void* B, int M, int N, int K, i
   if (choose && sym_mode == SYM_NONE && !ag_rows_per_rank && !col_scale && (!resid_f32 || (resid_f32 == out_f32 && !accumulate && !out_bf16))) {
     PairGemm g = {};
     g.A = A; g.B = B; g.M = M; g.N = N; g.K = K; g.lda = lda; g.ldb = ldb; g.out_f32 = out_f32; g.out_16 = out_bf16; g.half_out = half_out;
-    g.swiglu = act == ACT_SWIGLU_PAIR; g.add = accumulate || resid_f32; g.ldc = ldc; g.bias = bias; g.resid_bf16 = resid_bf16; g.alpha = alpha;
+    g.swiglu = act == ACT_SWIGLU_PAIR; g.add = out_f32 && (accumulate || resid_f32); g.ldc = ldc; g.bias = bias; g.resid_bf16 = resid_bf16; g.alpha = alpha;
     g.act = g.swiglu ? ACT_NONE : act; g.status = status;
     const long tiles = (long)((N + tile_n - 1) / tile_n) * tiles_m;
     if (choose_pair(g, tile_n, red_ok && tiles <= 74 ? (int)(148 / tiles) : 1)) return launch_gemm_pair(g, st);

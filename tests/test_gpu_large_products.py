@@ -72,6 +72,22 @@ def test_gemm_pair_refuses_what_it_cannot_store():
         ops.gemm_pair(A, B, 256, 256, 64, torch.empty((256, 257), device=DEV)[:, :256])
     with pytest.raises(RuntimeError):                              # splits add up: they need something to add to
         ops.gemm_pair(A, B, 256, 256, 64, torch.empty((256, 256), device=DEV), splits=2)
+    for splits in (1, 2):                                          # 16-bit results are stored, never added to
+        with pytest.raises(RuntimeError):
+            ops.gemm_pair(A, B, 256, 256, 64, torch.empty((256, 256), dtype=torch.bfloat16, device=DEV), add=True, splits=splits)
+
+
+@pytest.mark.parametrize("mn_major", [False, True])
+@pytest.mark.parametrize("M,N,K", [(256, 512, 4096), (2048, 4096, 512)])      # one that would split K, and one of many tiles
+def test_products_in_16_bits_are_whole_with_accumulate_set(M, N, K, mn_major):
+    """``accumulate`` adds to fp32 results; a 16-bit result is stored whole, flag or not."""
+    ops = _ops()
+    A, B = _randn(M, K, seed=50).bfloat16(), _randn(N, K, seed=51).bfloat16()
+    a, b = (A.t().contiguous(), B.t().contiguous()) if mn_major else (A, B)
+    out, status = torch.full((M, N), 3.0, dtype=torch.bfloat16, device=DEV), torch.zeros(1, dtype=torch.int32, device=DEV)
+    ops.gemm_bf16(a, b, M, N, K, lda=a.stride(0), ldb=b.stride(0), out_bf16=out, accumulate=True, mn_major=mn_major, status=status)
+    ref = A.float() @ B.float().t()
+    assert ((out.float() - ref).abs() <= _bound(A, B) + 2.0 ** -8 * ref.abs()).all() and int(status) == 0
 
 
 @pytest.mark.parametrize("T", [127, 128, 200])                     # either side of the row count where the kernel changes
