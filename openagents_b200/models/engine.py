@@ -3,7 +3,7 @@
 The engine owns the device weights, the paged fp16 KV cache and the activation workspaces, and runs the
 layers of the two operations ``PagedEngine`` exposes over packed token batches: ``forward_tokens`` (prefill
 chunks, many tokens per sequence) and ``decode`` (one token per sequence, replayed from a CUDA graph).  The weights stay
-in their packed GGUF block formats in device memory, once: one or two decode tokens take the quantized
+in their packed GGUF block formats in device memory, once: up to 4 decode tokens take the quantized
 mat-vec kernels (``dp4a``), up to 384 tokens the tcgen05 GEMM that expands the blocks inside its
 pipeline, and longer chunks (prefill) expand one matrix at a time into a scratch buffer for the
 bf16 tcgen05 GEMM.
@@ -75,11 +75,10 @@ class LlamaEngine(PagedEngine):
         self._init_paged(device, max_batch, max_ctx, n_pages, max_tokens, canaries)
         self._load(src)
         self._alloc()
-        # Up to this many decode tokens take the mat-vec path: its kernels scale with the token count, the tensor-core path does not.
-        # Measured on the 8B shape (ms per step, mat-vec / fused-dequant GEMM): 1 token 2.3 / 3.1, 2 tokens 2.9 / 3.1, 3 tokens
-        # 3.7 / 3.0, 8 tokens 5.0 / 3.0.  Weights which that GEMM does not take are expanded to bf16 first: mat-vec up to 4 tokens.
-        fused = self.world == 1 and all(self._qg(w) for l in self.layers for w in (l.wqkv, l.wo, l.wgu, l.wdown))
-        self.small_path_tokens = min(MATVEC_MAX_TOKENS, int(os.environ.get("B200_SMALL_PATH_TOKENS", 2 if fused else 4)))
+        # Up to this many decode tokens take the mat-vec path, which multiplies by the weights as they are packed (whole numbers times 32-bit
+        # scales); the fused-dequant GEMM rounds them to bf16.  Measured on the 8B shape (ms per step, mat-vec / GEMM): 1 token
+        # 2.3 / 3.1, 2 tokens 2.9 / 3.1, 3 tokens 3.7 / 3.0, 8 tokens 5.0 / 3.0: at 3 and 4 the difference buys the weights' precision.
+        self.small_path_tokens = min(MATVEC_MAX_TOKENS, int(os.environ.get("B200_SMALL_PATH_TOKENS", 4)))
         self.prefill_tc05 = os.environ.get("B200_PREFILL_TC05", "1") == "1"     # tcgen05 prefill attention (head sizes 64 and 128)
         self.seq_shard = os.environ.get("B200_TP_SEQ_SHARD", "1") == "1"        # sequence-sharded tensor-parallel prefill
         self.fuse_rope = os.environ.get("B200_FUSE_ROPE", "1") == "1"          # small-batch path: rotary + cache write in the QKV mat-vec
@@ -511,8 +510,9 @@ class LlamaEngine(PagedEngine):
         n = 2
         slots = self._slot_arg if self._slots_pending else None     # tensor parallel: the last layer's sum is still in the slots
         self._slots_pending = False
-        # The mat-vec takes 126 us for one row of the 8B head (Q6_K) and 242 for eight, the fused-dequant GEMM 130 for any number up to 64.
-        if nb <= (self.small_path_tokens if self._qg(self.wout) else MATVEC_MAX_TOKENS):
+        # Few rows: the mat-vec, with the weights as they are packed (126 us for one row of the 8B head in Q6_K, 242 for eight; the fused-dequant
+        # GEMM takes 130 for any number up to 64, but rounds them to bf16).
+        if nb <= MATVEC_MAX_TOKENS:
             q8 = self.wout.quantized
             ops.rmsnorm(rows, self.out_norm, cfg.norm_eps, xq=self.xq if q8 else None, xd=self.xd, xs16=self.xs,
                         hf=None if q8 else self.xf, slots=slots)

@@ -295,3 +295,21 @@ def test_scoring_on_the_engine_matches_the_cpu_backend(tmp_path):
     gpu.engine.check_status()
     assert all(abs(x - y) < 0.1 for x, y in zip(rg["picks"][0]["scores"], rc["picks"][0]["scores"]))
     assert gpu.kv_stats()["pages_free"] == free0                                 # every sequence was closed
+
+
+@pytest.mark.parametrize("batch,layers_fused", [(3, False), (4, False), (5, True), (8, True)])
+def test_few_decode_tokens_multiply_by_the_weights_as_packed(tmp_path, monkeypatch, batch, layers_fused):
+    """Up to four tokens no projection, and up to eight rows not the head, goes to the GEMM that rounds the weights to bf16."""
+    from openagents_b200.ops import cuda_ops as ops
+    cfg = TINY_LLAMA.with_(d_model=256, n_heads=4, n_kv_heads=2, head_dim=64, ffn=512, vocab=1024, n_layers=2)
+    p = str(tmp_path / "q4k.gguf")
+    save_gguf(p, cfg, random_weights(cfg, 3), PLAN_Q4_K)
+    eng = _engine(p)
+    for b in range(batch):
+        eng.begin(b)
+    eng.forward_tokens(list(range(batch)), [[1 + b, 2, 3] for b in range(batch)])
+    taken, real = [], ops.qgemm
+    monkeypatch.setattr(ops, "qgemm", lambda w, *a, **k: (taken.append(w), real(w, *a, **k))[1])
+    eng.decode(list(range(batch)), [7] * batch, use_graph=False)
+    assert not any(w is eng.wout for w in taken) and bool(taken) == layers_fused
+    eng.check_status()
