@@ -174,6 +174,7 @@ class LlamaEngine(PagedEngine):
         self.xs = ws("xs", (nb, kmax // 16 + 2), f32t)
         self.xf = ws("xf", (nb, kmax), f32t)
         # second activation set: a kernel never writes the buffers it is still reading
+        self.ff = ws("ff", (nb, F), f32t)          # not the rows of ``gu``: the fused GEMM's splits add into those and expect them cleared
         self.fq = ws("fq", (nb, kmax), i8)
         self.fd = ws("fd", (nb, kmax // 32 + 1), f32t)
         self.fs = ws("fs", (nb, kmax // 16 + 2), f32t)
@@ -318,19 +319,19 @@ class LlamaEngine(PagedEngine):
                         slots=self._slot_arg if slots else None)
             d8 = L.wdown.quantized and self.F % 32 == 0
             ops.matvec(L.wgu.wt, L.wgu.main, L.wgu.plane2, self.F, L.wgu.K, nb, xq=self.xq, xd=self.xd, xs16=self.xs,
-                       xf=self.xf, epi=ops.EPI_SWIGLU_Q8 if d8 else ops.EPI_SWIGLU_F32, y=self.gu, ldy=self.F,
+                       xf=self.xf, epi=ops.EPI_SWIGLU_Q8 if d8 else ops.EPI_SWIGLU_F32, y=self.ff, ldy=self.F,
                        oq=self.fq, od=self.fd, os16=self.fs)
             if not d8 and L.wdown.quantized:
-                ops.quantize_x(self.gu.view(-1)[: nb * self.F].view(nb, self.F), self.fq, self.fd, self.fs)
+                ops.quantize_x(self.ff[:nb], self.fq, self.fd, self.fs)
                 n += 1
             if self.world == 1:
                 ops.matvec(L.wdown.wt, L.wdown.main, L.wdown.plane2, L.wdown.N, L.wdown.K, nb, xq=self.fq, xd=self.fd,
-                           xs16=self.fs, xf=self.gu, epi=ops.EPI_RESID, resid=x, y=x, ldy=self.d)
+                           xs16=self.fs, xf=self.ff, epi=ops.EPI_RESID, resid=x, y=x, ldy=self.d)
             elif slots:
                 ops.matvec(L.wdown.wt, L.wdown.main, L.wdown.plane2, L.wdown.N, L.wdown.K, nb, xq=self.fq, xd=self.fd,
-                           xs16=self.fs, xf=self.gu, epi=ops.EPI_STORE, y=self.xpart, ldy=self.d)
+                           xs16=self.fs, xf=self.ff, epi=ops.EPI_STORE, y=self.xpart, ldy=self.d)
             else:
-                self.comm.matvec_allreduce(L.wdown, nb, self.fq, self.fd, self.fs, self.gu, x, self.d, wait_ready=not self._use_fence)
+                self.comm.matvec_allreduce(L.wdown, nb, self.fq, self.fd, self.fs, self.ff, x, self.d, wait_ready=not self._use_fence)
             n += 8
         self._slots_pending = slots          # the last down projection's sum is taken by the final norm
         return n

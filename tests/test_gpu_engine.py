@@ -313,3 +313,33 @@ def test_few_decode_tokens_multiply_by_the_weights_as_packed(tmp_path, monkeypat
     eng.decode(list(range(batch)), [7] * batch, use_graph=False)
     assert not any(w is eng.wout for w in taken) and bool(taken) == layers_fused
     eng.check_status()
+
+
+def test_short_prompts_after_decode_steps_with_an_unquantized_down_projection(tmp_path):
+    """Decode steps leave no gate/up values behind that a later prompt, whose splits add up in place, would add to."""
+    from openagents_b200.gguf import GgmlType
+    from openagents_b200.models.weights import QuantPlan
+
+    class Mixed(QuantPlan):
+        def type_for(self, spec):
+            return GgmlType.BF16 if "ffn_down" in spec.name else super().type_for(spec)
+
+    cfg = TINY_LLAMA.with_(d_model=256, n_heads=4, n_kv_heads=2, head_dim=64, ffn=512, vocab=1024, n_layers=2)
+    p = str(tmp_path / "mixed.gguf")
+    save_gguf(p, cfg, random_weights(cfg, 3), Mixed(matrix=PLAN_Q4_K.matrix, embed=PLAN_Q4_K.embed, output=PLAN_Q4_K.output))
+    eng = _engine(p)
+    g = torch.Generator().manual_seed(6)
+    for n in (40, 100):                                            # up to 64 tokens in all, and more
+        # the first rows of the batch are whole prompts, so that their logits show what was added to them
+        prompts = [torch.randint(0, cfg.vocab, (k,), generator=g).tolist() for k in (1, 1, 1, n)]
+        outs = []
+        for _ in range(2):
+            for b in range(4):
+                eng.begin(b)
+            outs.append(eng.forward_tokens(list(range(4)), prompts)[0].clone())
+            eng.decode(list(range(4)), [5, 6, 7, 8], use_graph=False)
+            for b in range(4):
+                eng.end(b)
+        # the same kernels on the same inputs; what differs is the order of the splits' 32-bit sums, and the bf16 roundings behind it
+        assert torch.allclose(*outs, atol=2e-2 * outs[0].std().item())
+    eng.check_status()
