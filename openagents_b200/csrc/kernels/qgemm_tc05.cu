@@ -56,6 +56,8 @@ struct QGemmArgs {
 __device__ __forceinline__ uint32_t bf162_as_u32(__nv_bfloat162 v) { return *reinterpret_cast<uint32_t*>(&v); }
 __device__ __forceinline__ __nv_bfloat162 u32_as_bf162(uint32_t v) { return *reinterpret_cast<__nv_bfloat162*>(&v); }
 
+__device__ __forceinline__ float low_half(uint32_t t) { return __uint_as_float(t << 16); }
+__device__ __forceinline__ float high_half(uint32_t t) { return __uint_as_float(t & 0xFFFF0000u); }
 __device__ __forceinline__ uint32_t pack2(float lo, float hi) { return bf162_as_u32(__floats2bfloat162_rn(lo, hi)); }
 
 // Q4_K-R: one 32-element sub-block (4 words, word w = elements 8w .. 8w + 7, element i at bit
@@ -64,10 +66,11 @@ __device__ __forceinline__ uint32_t pack2(float lo, float hi) { return bf162_as_
 // the constant small (the sub-block's range is roughly centred on it), so rounding a and c to bf16 costs no more
 // than rounding the weight itself does.
 //
-// FINE: the scale in two bf16 parts (one more fma a pair) and, in place of 8, the whole number n nearest to min / a, so that the
-// constant is at most half a step.  What is left is the result's own rounding, the one that dequant.cu makes.
-template <bool FINE>
-__device__ __forceinline__ void expand_q4k(__nv_bfloat162 off, __nv_bfloat162 A2, __nv_bfloat162 A2lo, __nv_bfloat162 C2, const uint4 q, uint32_t* out) {
+// WHOLE: the weight itself in 32 bits, rounded to bf16 once: the value that dequant.cu makes, bit for bit (`scale` and `least` are the
+// sub-block's 32-bit scale and min, `A2` and `C2` unused).
+template <bool WHOLE>
+__device__ __forceinline__ void expand_q4k(__nv_bfloat162 A2, __nv_bfloat162 C2, float scale, float least, const uint4 q, uint32_t* out) {
+  const __nv_bfloat162 off = __halves2bfloat162(__float2bfloat16(WHOLE ? 16.f : 24.f), __float2bfloat16(WHOLE ? 16.f : 24.f));
   const uint32_t w[4] = {q.x, q.y, q.z, q.w};
 #pragma unroll
   for (int i = 0; i < 4; i++) {
@@ -78,7 +81,9 @@ __device__ __forceinline__ void expand_q4k(__nv_bfloat162 off, __nv_bfloat162 A2
     const uint32_t t3 = ((v >> 9) & 0x00780078u) | 0x41804180u;
     auto finish = [&](uint32_t t) {
       const __nv_bfloat162 x = __hsub2(u32_as_bf162(t), off);
-      return bf162_as_u32(__hfma2(x, A2, FINE ? __hfma2(x, A2lo, C2) : C2));
+      if constexpr (!WHOLE) return bf162_as_u32(__hfma2(x, A2, C2));
+      const uint32_t u = bf162_as_u32(x);
+      return pack2(fmaf(scale, low_half(u), -least), fmaf(scale, high_half(u), -least));
     };
     out[4 * i + 0] = finish(t0);
     out[4 * i + 1] = finish(t1);
@@ -87,11 +92,11 @@ __device__ __forceinline__ void expand_q4k(__nv_bfloat162 off, __nv_bfloat162 A2
   }
 }
 
-// Q6_K-R: 6-bit value = nibble | two high bits; (64 + q) - 96 = q - 32 is exact in bf16.  `ss` holds
-// the two bf16 scales of the sub-block (first and second 16 elements); FINE: `ss_lo` what their rounding left.
-template <bool FINE>
-__device__ __forceinline__ void expand_q6k(const uint4 lo, const uint2 tw, uint32_t ss, uint32_t ss_lo, uint32_t* out) {
-  const __nv_bfloat162 sv = u32_as_bf162(ss), sl = u32_as_bf162(ss_lo);
+// Q6_K-R: 6-bit value = nibble | two high bits; (64 + q) - 96 = q - 32 is exact in bf16.  `s0` and `s1` are the scales of the
+// sub-block's first and second 16 elements, rounded to bf16 here unless WHOLE.
+template <bool WHOLE>
+__device__ __forceinline__ void expand_q6k(const uint4 lo, const uint2 tw, float s0, float s1, uint32_t* out) {
+  const __nv_bfloat162 sv = __floats2bfloat162_rn(s0, s1);
   const __nv_bfloat162 off = __halves2bfloat162(__float2bfloat16(96.f), __float2bfloat16(96.f));
   const uint32_t w[4] = {lo.x, lo.y, lo.z, lo.w};
 #pragma unroll
@@ -99,10 +104,12 @@ __device__ __forceinline__ void expand_q6k(const uint4 lo, const uint2 tw, uint3
     const uint32_t v = w[i];
     const uint32_t T = (i < 2 ? tw.x : tw.y) >> (4 * (i & 1));
     const __nv_bfloat162 S2 = i < 2 ? __halves2bfloat162(sv.x, sv.x) : __halves2bfloat162(sv.y, sv.y);
-    const __nv_bfloat162 L2 = i < 2 ? __halves2bfloat162(sl.x, sl.x) : __halves2bfloat162(sl.y, sl.y);
+    const float scale = i < 2 ? s0 : s1;
     auto finish = [&](uint32_t q) {
       const __nv_bfloat162 x = __hsub2(u32_as_bf162((q << 1) | 0x42804280u), off);
-      return bf162_as_u32(FINE ? __hfma2(x, S2, __hmul2(x, L2)) : __hmul2(x, S2));
+      if constexpr (!WHOLE) return bf162_as_u32(__hmul2(x, S2));
+      const uint32_t u = bf162_as_u32(x);
+      return pack2(scale * low_half(u), scale * high_half(u));
     };
     const uint32_t q0 = (v & 0x000F000Fu) | ((T & 0x00030003u) << 4);
     const uint32_t q1 = ((v >> 4) & 0x000F000Fu) | (((T >> 2) & 0x00030003u) << 4);
@@ -190,7 +197,9 @@ __global__ void __launch_bounds__(kQThreads, 1) qgemm_kernel(const __grid_consta
   const uint32_t tmem_base = *tmem_holder;
   // tensor-memory columns: accumulators at +0 and +QBN, then operand stages of 128 columns (256 of K) each
   constexpr uint32_t kOpCol = 2 * QBN;
-  constexpr bool kFine = QBN == 128;      // prompts: their weights are not rounded more often than by the expansion that longer ones take
+  // More than 64 tokens: the weights that the expansion for longer prompts gives.  In 32 bits a pair takes eight instructions in place of four (an 8B prompt of
+  // 128 tokens takes 4.2 ms, 4.0 with scales in two bf16 parts, 8.3 through the expansion).
+  constexpr bool kWhole = QBN == 128;
   pdl_trigger();
 
   if (warp == 0) {
@@ -409,23 +418,18 @@ __global__ void __launch_bounds__(kQThreads, 1) qgemm_kernel(const __grid_consta
             for (int h = 0; h < 2; h++) {
               const int j = 2 * kbu + h, sh = 8 * (j & 3);
               const float av = d4 * (float)((S >> sh) & 0xFFu);
-              const __nv_bfloat16 ab = __float2bfloat16(av);
-              const __nv_bfloat16 al = __float2bfloat16(av - __bfloat162float(ab));
               const float least = dmin4 * (float)((Mn >> sh) & 0xFFu);
-              const float n8 = kFine ? fminf(fmaxf(rintf(__fdividef(least, av)), 0.f), 15.f) : 8.f;
-              const __nv_bfloat16 cb = __float2bfloat16(n8 * (kFine ? av : __bfloat162float(ab)) - least), off = __float2bfloat16(16.f + n8);
-              expand_q4k<kFine>(__halves2bfloat162(off, off), __halves2bfloat162(ab, ab), __halves2bfloat162(al, al), __halves2bfloat162(cb, cb),
-                                *(const uint4*)(rowp + 16 + j * 16), r + 16 * h);
+              const __nv_bfloat16 ab = __float2bfloat16(av);
+              const __nv_bfloat16 cb = __float2bfloat16(8.f * __bfloat162float(ab) - least);
+              expand_q4k<kWhole>(__halves2bfloat162(ab, ab), __halves2bfloat162(cb, cb), av, least, *(const uint4*)(rowp + 16 + j * 16), r + 16 * h);
             }
           } else {
 #pragma unroll
             for (int h = 0; h < 2; h++) {
               const int j = 2 * kbu + h;
               const uint32_t scw = *(const uint16_t*)(rowp + 192 + 2 * j);
-              const float s0 = d6 * (float)(int8_t)(scw & 0xFF), s1 = d6 * (float)(int8_t)(scw >> 8);
-              const __nv_bfloat162 ss = __floats2bfloat162_rn(s0, s1);
-              const __nv_bfloat162 sl = __floats2bfloat162_rn(s0 - __bfloat162float(ss.x), s1 - __bfloat162float(ss.y));
-              expand_q6k<kFine>(*(const uint4*)(rowp + j * 16), *(const uint2*)(rowp + 128 + j * 8), bf162_as_u32(ss), bf162_as_u32(sl), r + 16 * h);
+              expand_q6k<kWhole>(*(const uint4*)(rowp + j * 16), *(const uint2*)(rowp + 128 + j * 8), d6 * (float)(int8_t)(scw & 0xFF),
+                                 d6 * (float)(int8_t)(scw >> 8), r + 16 * h);
             }
           }
           if (u == 0) {      // the first values are in registers: only now does this warp need the operand slot

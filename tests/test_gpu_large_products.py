@@ -223,6 +223,23 @@ def test_fused_dequant_gemm_of_short_prompts(kind, T, N, K):
     assert int(status) == 0
 
 
+@pytest.mark.parametrize("kind", ["Q4_K", "Q6_K"])
+@pytest.mark.parametrize("spread", [1.0, 30.0])                    # weights of one size, and heavy tails inside every block
+def test_fused_dequant_gemm_of_short_prompts_rounds_weights_once(kind, spread):
+    """One-hot rows give the weights themselves: the very ones of the bf16 expansion, in every row and superblock."""
+    from openagents_b200.gguf import GgmlType
+    from openagents_b200.gguf import torch_codecs as tc
+    from openagents_b200.models.qweight import QWeight, RawTensor
+    ops, t, N, K = _ops(), GgmlType[kind], 392, 1280
+    weights = _randn(N, K, seed=33) * 0.02 * spread ** _randn(N, K, seed=34).clamp(-2, 2)
+    weights[5] = 0.0
+    weights[6, :512] = weights[6, :512].abs() + 0.5
+    w = QWeight.from_raw(RawTensor(t, (N, K), tc.quantize(weights, t)))
+    y, status = torch.empty((K, N), device=DEV), torch.zeros(1, dtype=torch.int32, device=DEV)
+    ops.qgemm(w, torch.eye(K, device=DEV).bfloat16(), K, out_f32=y, epi=ops.QEPI_STORE, status=status)
+    assert torch.equal(y.t(), w.dequant_into(torch.empty((N, K), dtype=torch.bfloat16, device=DEV)).float()) and int(status) == 0
+
+
 @pytest.mark.parametrize("D", [64, 256, 264, 512, 768, 776, 1024, 1032])      # either side of every width that a row in registers is built for
 @pytest.mark.parametrize("rows,add", [(5, False), (3000, True)])
 def test_layernorm_backward_widths(D, rows, add):
