@@ -14,7 +14,7 @@ A layer's feed-forward block is three kernels:
    ends with the cross-rank barrier.  There is no separate combine or all-to-all launch.
 
 Expert weights arrive as MXFP4 blocks (GGUF) and are expanded once, at load, to bf16 for the tensor
-cores; the expansion is exact.  On one rank the packed blocks are kept beside it (a quarter more): a
+cores; the expansion is exact.  On one rank the packed blocks are kept beside it where memory allows (a quarter more): a
 step with few rows per expert reads those and expands them inside the GEMM (``moe_qgemm.cu``).
 
 The reference names this topology without implementing it: ``sparse_expert`` placement with
@@ -35,6 +35,7 @@ from ..ops import cuda_ops as ops
 from ..parallel.tp import TPComm
 from .config import ModelConfig
 from .engine import LlamaEngine, _Layer
+from .paged import PAGE
 from .qweight import RawTensor, WeightSource
 from ..utils.nvtx import nvtx_method
 
@@ -69,6 +70,18 @@ class MoEEngine(LlamaEngine):
         self.small_path_tokens = 0                                   # every batch size takes the tensor-core path
 
     # ------------------------------------------------------------------ weights
+    def _packed_fit(self) -> bool:
+        """Whether the packed blocks (17/32 of a byte a weight, beside two of its expansion) fit the device with all that the engine needs anyway:
+        an engine that fits without them is not refused for their sake.  A twentieth of the memory is left for what loading a layer takes."""
+        cfg = self.cfg
+        experts = cfg.n_layers * 3 * self.E_local * cfg.ffn * cfg.d_model
+        others = cfg.n_layers * 2 * cfg.d_model * (cfg.q_dim + cfg.kv_dim) + 2 * cfg.vocab * cfg.d_model
+        cache = cfg.n_layers * 2 * self.n_pages * PAGE * cfg.kv_dim * 2
+        rows = self.E_local * self.cap * cfg.ffn * 2 + self.max_tokens * (14 * cfg.d_model + 8 * (cfg.q_dim + cfg.kv_dim) + 12 * cfg.ffn)
+        free, total = torch.cuda.mem_get_info(self.device)
+        free += torch.cuda.memory_reserved(self.device) - torch.cuda.memory_allocated(self.device)
+        return free - (experts * (2 + 17 / 32) + 2 * others + cache + rows + self.max_batch * cfg.vocab * 4) > total / 20
+
     def _load_ffn(self, src: WeightSource, p: str, layer: int):
         e0, e1 = self.ep_rank * self.E_local, (self.ep_rank + 1) * self.E_local
         f, d = self.cfg.ffn, self.cfg.d_model
@@ -78,7 +91,9 @@ class MoEEngine(LlamaEngine):
         del g, u
         w2 = rd.to_float().view(self.E_local * d, f).to(torch.bfloat16).contiguous()
         q13 = q2 = None
-        if self.ep_world == 1 and all(r.type == GgmlType.MXFP4 for r in (rg, ru, rd)):
+        if layer == 0:
+            self._keep_packed = self.ep_world == 1 and self._packed_fit()
+        if self._keep_packed and all(r.type == GgmlType.MXFP4 for r in (rg, ru, rd)):
             pairs = RawTensor.interleave_rows(*(RawTensor(r.type, (self.E_local * f, d), r.data) for r in (rg, ru)))
             q13, q2 = tc.pack_mxfp4_wide(pairs.data.to(w2.device), 2 * f * self.E_local), tc.pack_mxfp4_wide(rd.data.to(w2.device), d * self.E_local)
             if q13 is None or q2 is None:

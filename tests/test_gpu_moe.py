@@ -131,3 +131,20 @@ def test_moe_ffn_block_of_many_rows_matches_oracle(tmp_path):
             err = (x.cpu() - ref).abs().max().item()
             assert err < 0.03 * ref.abs().max().item() + 1e-4, (T, li, err, ref.abs().max().item())
     eng.check_status()
+
+
+def test_moe_engine_without_room_for_the_packed_experts(tmp_path, monkeypatch):
+    """Where memory is short the engine loads without the packed blocks and serves from the bf16 expansion."""
+    from openagents_b200.models.moe_engine import MoEEngine
+    from openagents_b200.models.qweight import GGUFSource
+    p = _make(tmp_path)
+    cfg2, W = load_gguf_float(p)
+    with monkeypatch.context() as m:
+        m.setattr(torch.cuda, "mem_get_info", lambda *a: (8 << 30, 180 << 30))      # enough for this model, less than the margin
+        src = GGUFSource(p, "cuda")
+        eng = MoEEngine(src.cfg, src, max_batch=8, max_ctx=128, max_tokens=256)
+    assert all(e.q13 is None and e.q2 is None for e in eng.experts)
+    _check_against_oracle(eng, cfg2, W, _prompts(3, 1))
+    roomy = MoEEngine(src.cfg, GGUFSource(p, "cuda"), max_batch=8, max_ctx=128, max_tokens=256)
+    assert all(e.q13 is not None and e.q2 is not None for e in roomy.experts)
+    assert roomy.weight_bytes() - eng.weight_bytes() == cfg2.n_layers * 3 * cfg2.n_experts * cfg2.ffn * cfg2.d_model * 17 // 32
