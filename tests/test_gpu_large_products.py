@@ -257,3 +257,139 @@ def test_layernorm_backward_widths(D, rows, add):
     assert ((dx.double() - want).abs() <= 2.0 ** -8 * want.abs() + 1e-4).all()
     for got, ref in ((dg, gr.grad), (db, br.grad)):      # sums of `rows` terms of size about one to ten in 32 bits
         assert ((got.double() - ref).abs() <= 2.0 ** -18 * rows + 1e-4).all()
+
+
+def _pair_sizes_inplace(ops, M, N, K, how):
+    A, B, x0, bias = _randn(M, K, seed=60).bfloat16(), _randn(N, K, seed=61).bfloat16(), _randn(M, N, seed=62), _randn(N, seed=63)
+    x, status = x0.clone(), torch.zeros(1, dtype=torch.int32, device=DEV)
+    ops.gemm_bf16(A, B, M, N, K, out_f32=x, bias=bias, resid_f32=x if how == "resid" else None, accumulate=how == "accumulate", status=status)
+    return (x - (x0 + A.float() @ B.float().t() + bias)).abs() <= _bound(A, B) + 1e-5, int(status)
+
+
+@pytest.mark.parametrize("how", ["resid", "accumulate"])
+@pytest.mark.parametrize("M,N,K", [(2048, 4096, 512), (300, 2048, 4096), (1000, 4100, 776)])      # many tiles; few, with K split; tiles that end inside
+def test_large_products_added_in_place(M, N, K, how):
+    ok, status = _pair_sizes_inplace(_ops(), M, N, K, how)
+    assert ok.all() and status == 0
+
+
+# more than 128 rows an expert on average; a group of an odd number of 128-row tiles, so that a pair's tile ends in the next one's rows; experts
+# without rows, with one, with all; several stages of K with a remainder; columns that end inside a tile
+@pytest.mark.parametrize("counts,K,f,d", [((0, 1, 129, 257, 384, 384), 200, 160, 328), ((384,), 712, 144, 64), ((256, 131, 384), 64, 512, 768)])
+def test_expert_products_of_many_rows(counts, K, f, d):
+    ops, E, cap = _ops(), len(counts), 384
+    x, w13 = _randn(E * cap, K, seed=64).bfloat16(), _randn(E * 2 * f, K, seed=65).bfloat16() * 0.1
+    cnt, rows = torch.tensor(counts, dtype=torch.int32, device=DEV), sum(counts)
+    assert rows > 128 * E
+    gate, status = torch.rand(E * cap, device=DEV) + 0.5, torch.zeros(1, dtype=torch.int32, device=DEV)
+    live = torch.cat([torch.arange(c, device=DEV) + e * cap for e, c in enumerate(counts)])
+    for w in (None, gate):                                         # a weight multiplies the expert's input
+        mid = torch.full((E * cap, f), 7.0, dtype=torch.bfloat16, device=DEV)
+        ops.moe_gemm(x, w13, E, cap, 2 * f, K, cnt, 1, out_bf16=mid, ldc=f, gate_w=w, live_rows=rows, status=status)
+        for e, c in enumerate(counts):
+            s = slice(e * cap, e * cap + c)
+            scale = 1.0 if w is None else w[s, None]
+            gu, mag = scale * (x[s].float() @ w13[e * 2 * f:(e + 1) * 2 * f].float().t()), scale * (x[s].float().abs() @ w13[e * 2 * f:(e + 1) * 2 * f].float().abs().t())
+            want = torch.nn.functional.silu(gu[:, 0::2]) * gu[:, 1::2]
+            tol = 2.0 ** -17 * 1.1 * (mag[:, 0::2] * (gu[:, 1::2].abs() + 1) + mag[:, 1::2] * gu[:, 0::2].abs()) + (2.0 ** -8 + 2.0 ** -10) * want.abs() + 1e-5
+            assert ((mid[s].float() - want).abs() <= tol).all(), e
+            assert (mid[e * cap + -(-c // 32) * 32:(e + 1) * cap] == 7.0).all(), e        # the patch of 32 rows that holds the last one, and no further
+    h, w2 = _randn(E * cap, K, seed=66).bfloat16(), _randn(E * d, K, seed=67).bfloat16()
+    tokens = torch.randperm(E * cap, generator=torch.Generator().manual_seed(68)).to(DEV) % 500
+    meta = torch.stack((torch.zeros_like(tokens), tokens), 1).int().contiguous()
+    for w in (None, gate):
+        y0 = _randn(500, d, seed=69)
+        y = y0.clone()
+        ops.moe_gemm(h, w2, E, cap, d, K, cnt, 2, ldc=d, meta=meta, gate_w=w, sym_off=y.data_ptr(), live_rows=rows, status=status)
+        ref, scale = y0.double(), y0.double().abs()
+        per_row = torch.cat([h[e * cap:e * cap + c].double() @ w2[e * d:(e + 1) * d].double().t() for e, c in enumerate(counts)])
+        mags = torch.cat([h[e * cap:e * cap + c].double().abs() @ w2[e * d:(e + 1) * d].double().t().abs() for e, c in enumerate(counts)])
+        g = torch.ones(rows, 1, device=DEV).double() if w is None else w[live, None].double()
+        ref.index_add_(0, tokens[live], g * per_row)
+        scale.index_add_(0, tokens[live], g * mags)
+        assert ((y - ref).abs() <= 2.0 ** -17 * scale).all()
+    assert int(status) == 0
+
+
+@pytest.mark.parametrize("T", [295, 296, 297, 298, 592, 593, 4096])      # from 297 tokens on a CTA takes two of them, the last one what is left
+@pytest.mark.parametrize("E,d,top_k", [(32, 2880, 4), (5, 72, 2)])
+def test_routing_of_many_tokens(T, E, d, top_k):
+    ops = _ops()
+    h32, wr, br = _randn(T, d, seed=70), _randn(E, d, seed=71) / d ** 0.5, _randn(E, seed=72)
+    h = h32.bfloat16()
+    recv, meta = torch.full((E * T, d), 9.0, dtype=torch.bfloat16, device=DEV), torch.full((E * T, 2), -1, dtype=torch.int32, device=DEV)
+    weight, counts = torch.zeros(E * T, device=DEV), torch.zeros(E, dtype=torch.int32, device=DEV)
+    ids, w = torch.empty((T, top_k), dtype=torch.int32, device=DEV), torch.empty((T, top_k), device=DEV)
+    status = torch.zeros(1, dtype=torch.int32, device=DEV)
+    ops.moe_route_dispatch(h, h32, wr, br, top_k, E, T, *(t.data_ptr() for t in (recv, meta, weight, counts)), None, topk_ids=ids, topk_w=w, status=status)
+    one_i, one_w = torch.empty_like(ids), torch.empty_like(w)
+    for lo in range(0, T, 250):                                    # the form of one token a CTA
+        s = slice(lo, min(T, lo + 250))
+        ops.moe_route_dispatch(None, h32[s], wr, br, top_k, E, 0, 0, 0, 0, 0, None, topk_ids=one_i[s], topk_w=one_w[s])
+    logits = h32.double() @ wr.double().t() + br.double()
+    tol = 2.0 ** -20 * (h32.double().abs() @ wr.double().abs().t() + br.double().abs()).max()
+    # the chosen are the largest but for ties within the sums' error, in either form
+    for i, v in ((ids, w), (one_i, one_w)):
+        chosen = logits.gather(1, i.long())
+        assert (logits.topk(top_k, 1).values - chosen).abs().max() <= 2 * tol
+        assert torch.allclose(v.double(), torch.softmax(chosen, 1), atol=1e-5)
+    assert (ids == one_i).float().mean() > 0.999
+    assert torch.equal(counts.long(), torch.bincount(ids.flatten().long(), minlength=E)) and int(status) == 0
+    for e in range(E):
+        n = int(counts[e])
+        s = slice(e * T, e * T + n)
+        t = meta[s, 1].long()
+        assert (meta[s, 0] == 0).all() and torch.equal(t.sort().values, (ids == e).any(1).nonzero().flatten())
+        assert torch.equal(recv[s], h[t]) and torch.equal(weight[s], w[t][ids[t] == e])
+        assert (recv[s.stop:(e + 1) * T] == 9.0).all()
+
+
+@pytest.mark.parametrize("window,use_sinks", [(0, True), (1024, True), (1056, False), (0, False)])
+def test_prefill_attention_of_head_size_64(window, use_sinks):
+    """Head size 64 on tcgen05, with the long windows and sinks it takes there: cold prompts, chunks behind a context, one token, ends inside a block."""
+    from test_gpu_kernels import _paged_kv
+
+    from openagents_b200.oracle import nn
+    ops, hd, Hq, Hkv = _ops(), 64, 8, 2
+    ctx, qlen = [1500, 1217, 129, 2050], [1500, 64, 1, 257]
+    kc, vc, table, Ks, Vs = _paged_kv(4, Hkv, hd, ctx, seed=73)
+    starts = [sum(qlen[:b]) for b in range(4)]
+    q = (_randn(sum(qlen), Hq * hd, seed=74) * (3.0 / hd ** 0.5)).half()
+    sinks = _randn(Hq, seed=75) if use_sinks else None
+    out, status = torch.zeros((sum(qlen), Hq * hd), dtype=torch.bfloat16, device=DEV), torch.zeros(1, dtype=torch.int32, device=DEV)
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)
+    ops.attn_prefill_tc05(q, kc, vc, table, i32(starts), i32(qlen), i32(ctx), 4, max(qlen), Hq, Hkv, window=window, sinks=sinks, out_bf16=out,
+                          status=status, dk=hd, dv=hd)
+    assert int(status) == 0
+    for b in range(4):
+        s, n = starts[b], qlen[b]
+        ref = nn.attention(q[s:s + n].float().cpu().view(n, Hq, hd), Ks[b], Vs[b], torch.arange(ctx[b] - n, ctx[b]), torch.arange(ctx[b]),
+                           window=window, sinks=None if sinks is None else sinks.cpu(), scale=1.0).reshape(n, -1)
+        # probabilities in 16 bits (2^-11 of values of size about one, averaged) and the result in bf16
+        assert ((out[s:s + n].float().cpu() - ref).abs() <= 2.0 ** -8 * ref.abs() + 4e-3).all(), b
+
+
+# K of one K block, of a two-block stage and a half, of a ring that just fits, wraps, and wraps with a remainder; columns for tiles of 64, 128 and 256
+@pytest.mark.parametrize("M", [1, 7, 33, 64])
+@pytest.mark.parametrize("K", [64, 72, 192, 768, 1032, 4104])
+@pytest.mark.parametrize("N,add", [(192, False), (192, True), (2304, True), (14848, False), (28672, False)])
+def test_few_row_products_with_weights_loaded_ahead(M, K, N, add):
+    """``b_ready`` moves loads of B ahead of the wait for the kernel before; A is written by that very kernel."""
+    ops = _ops()
+    src, B, x0 = _randn(M, K, seed=76), _randn(N, K, seed=77).bfloat16(), _randn(M, N, seed=78)
+    gain, status = torch.ones(K, device=DEV), torch.zeros(1, dtype=torch.int32, device=DEV)
+    if K % 32:                                                     # the norm takes rows of whole 32s: the same values by a plain copy
+        write = lambda A: A.copy_(src)
+    else:
+        write = lambda A: ops.rmsnorm(src, gain, 1e-5, hb=A)
+    outs = []
+    for ready in (True, False):
+        A = torch.full((M, K), float("nan"), dtype=torch.bfloat16, device=DEV)      # what a load ahead of the wait would bring
+        out = x0.clone() if add else torch.empty((M, N), device=DEV)
+        torch.cuda.synchronize()
+        write(A)
+        ops.gemm_bf16(A, B, M, N, K, out_f32=out, accumulate=add, b_ready=ready, status=status)
+        outs.append(out)
+    tol = _bound(A, B) + 1e-5
+    assert ((outs[0] - outs[1]).abs() <= 2 * tol).all()
+    assert ((outs[0] - A.float() @ B.float().t() - (x0 if add else 0)).abs() <= tol).all() and int(status) == 0

@@ -148,3 +148,28 @@ def test_moe_engine_without_room_for_the_packed_experts(tmp_path, monkeypatch):
     roomy = MoEEngine(src.cfg, GGUFSource(p, "cuda"), max_batch=8, max_ctx=128, max_tokens=256)
     assert all(e.q13 is not None and e.q2 is not None for e in roomy.experts)
     assert roomy.weight_bytes() - eng.weight_bytes() == cfg2.n_layers * 3 * cfg2.n_experts * cfg2.ffn * cfg2.d_model * 17 // 32
+
+
+def test_moe_ffn_block_of_many_rows_matches_oracle(tmp_path):
+    """More rows an expert than the packed weights serve: the bf16 expansion, on single CTAs and (above 128 rows an expert) on pairs."""
+    from openagents_b200.models.moe_engine import MoEEngine
+    from openagents_b200.models.qweight import GGUFSource
+    from openagents_b200.ops import cuda_ops as ops
+    from openagents_b200.oracle.models import moe_ffn
+    p = _make(tmp_path)
+    cfg2, W = load_gguf_float(p)
+    src = GGUFSource(p, "cuda")
+    eng = MoEEngine(src.cfg, src, max_batch=8, max_ctx=128, max_tokens=1024)
+    for T in (256, 257, 512, 513, 1000):                           # 64, 64.25, 128, 128.25 and 250 rows an expert on average
+        hb = torch.randn(T, cfg2.d_model, generator=torch.Generator().manual_seed(T)).bfloat16().cuda()
+        eng.hf32[:T].copy_(hb.float())
+        x = eng.x[:T]
+        for li in (0, 1):
+            ops.moe_zero(eng.counts)
+            x.zero_()
+            eng._ffn_dense(li, eng.layers[li], T, x, hb, None, None)
+            ref = moe_ffn(cfg2, W, f"blk.{li}.", hb.float().cpu())
+            assert int(eng.counts[li & 1].sum()) == T * cfg2.top_k
+            err = (x.cpu() - ref).abs().max().item()
+            assert err < 0.03 * ref.abs().max().item() + 1e-4, (T, li, err, ref.abs().max().item())
+    eng.check_status()
