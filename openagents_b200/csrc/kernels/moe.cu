@@ -1,6 +1,6 @@
 // Mixture-of-experts routing fused with the expert-parallel dispatch.
 //
-// One CTA per token or four tokens: router logits (an [E][d] fp32 mat-vec against the normalised hidden row), top-k,
+// One CTA per token or two tokens: router logits (an [E][d] fp32 mat-vec against the normalised hidden row), top-k,
 // softmax over the selected k (the gpt-oss convention), and then, for each selected expert, the row is
 // written straight into the receive buffer of the rank that owns the expert: a slot is claimed with
 // one atomic on the owner's counter and the 16-byte stores go over NVLink peer memory (or stay local).
@@ -64,7 +64,7 @@ __global__ void __launch_bounds__(256, TPC == 1 ? 1 : 4) moe_route_dispatch_kern
 #pragma unroll
       for (int j = 0; j < 4; j++) acc[t][j] = 0.f;
     if constexpr (WIDE) {
-#pragma unroll(TPC == 1 ? 4 : 1)      // four tokens: CTAs in flight instead of iterations
+#pragma unroll(TPC == 1 ? 4 : 2)      // two tokens: CTAs in flight instead of iterations
       for (int i = lane * 4; i < a.d; i += 128) {
         float4 y[4];
 #pragma unroll
@@ -169,19 +169,19 @@ __global__ void __launch_bounds__(256, TPC == 1 ? 1 : 4) moe_route_dispatch_kern
   if (!a.dispatch) return;
   __syncthreads();
 
-  // Copy the rows to each owner, 16 bytes per thread per step (d * 2 bytes is a multiple of 16).
+  // Copy the rows to each owner, 16 bytes per thread per step (d * 2 bytes is a multiple of 16), the tokens' rows as one run.
   const int n16 = a.d / 8;
-  for (int t = 0; t < live; t++) {
-    const uint4* src = (const uint4*)(a.h + (size_t)(t0 + t) * a.d);
-    for (int i = tid; i < n16; i += 256) {
-      const uint4 v = src[i];
-      for (int k = 0; k < a.top_k; k++) {
-        if (s_slot[t][k] < 0) continue;
-        const int owner = s_sel[t][k] / a.E_local, el = s_sel[t][k] % a.E_local;
-        char* dst = a.sym.base[owner] + a.recv_x_off + ((size_t)el * a.C + s_slot[t][k]) * (size_t)a.d * 2;
-        asm volatile("st.relaxed.sys.global.v4.u32 [%0], {%1,%2,%3,%4};" ::"l"(dst + (size_t)i * 16), "r"(v.x), "r"(v.y),
-                     "r"(v.z), "r"(v.w) : "memory");
-      }
+  const uint4* src = (const uint4*)(a.h + (size_t)t0 * a.d);
+#pragma unroll 2
+  for (int i = tid; i < live * n16; i += 256) {
+    const int t = TPC == 1 ? 0 : i / n16, c = i - t * n16;
+    const uint4 v = src[i];
+    for (int k = 0; k < a.top_k; k++) {
+      if (s_slot[t][k] < 0) continue;
+      const int owner = s_sel[t][k] / a.E_local, el = s_sel[t][k] % a.E_local;
+      char* dst = a.sym.base[owner] + a.recv_x_off + ((size_t)el * a.C + s_slot[t][k]) * (size_t)a.d * 2 + (size_t)c * 16;
+      if (a.local) *(uint4*)dst = v;
+      else asm volatile("st.relaxed.sys.global.v4.u32 [%0], {%1,%2,%3,%4};" ::"l"(dst), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
     }
   }
   if (!a.local) sym_kernel_end_barrier(a.sym, 3, gridDim.x);
@@ -211,10 +211,12 @@ B200_API int b200_moe_route_dispatch(const void* h, const float* hf, const float
   a.local = !sym;
   if (sym) a.sym = *sym;
   else a.sym = SymTable{};
-  // Four tokens a CTA once that still leaves every SM several CTAs.  32 experts of 2880, top 4, with the copies: 256 tokens 36 -> 18 us, 4096 tokens 150 -> 103.
+  // One token a CTA while the two CTAs that an SM holds of that form take all of them at once, else two (four CTAs an SM).  32 experts of
+  // 2880, top 4, us with the copies, one / two: 296 tokens 10.1 / 12.7, 300 tokens 16.0 / 13.7, 800 tokens 26.7 / 19.6, 4096 tokens 149 / 94
+  // (112 with four tokens a CTA, which takes 31 for 800).
   if (((uintptr_t)wr | (uintptr_t)hf | (uintptr_t)h) & 15) return launch_pdl(moe_route_dispatch_kernel<1, false>, dim3(T), dim3(256), 0, st, a);
-  if (T < 4 * 148) return launch_pdl(moe_route_dispatch_kernel<1, true>, dim3(T), dim3(256), 0, st, a);
-  return launch_pdl(moe_route_dispatch_kernel<4, true>, dim3((T + 3) / 4), dim3(256), 0, st, a);
+  if (T <= 2 * 148) return launch_pdl(moe_route_dispatch_kernel<1, true>, dim3(T), dim3(256), 0, st, a);
+  return launch_pdl(moe_route_dispatch_kernel<2, true>, dim3((T + 1) / 2), dim3(256), 0, st, a);
 }
 
 // ------------------------------------------------------------------ chosen experts of few tokens, and experts in 32-bit
