@@ -45,21 +45,6 @@ __device__ __forceinline__ float exp_scale(float m, float M) {
   return m == -INFINITY ? 0.f : __expf(m - M);
 }
 
-template <int DV>
-__device__ __forceinline__ void write_out(const AttnDecArgs& a, int b, int h, int e, float o) {
-  const int col = h * DV + e;
-  const size_t row = (size_t)b * a.Hq * DV;
-  if (a.out_f32) a.out_f32[row + col] = o;
-  if (a.out_bf16) a.out_bf16[row + col] = __float2bfloat16(o);
-  if (a.oq) {
-    const int lane = threadIdx.x & 31;
-    const int blk = col >> 5;
-    const size_t nblk = (size_t)a.Hq * DV / 32;
-    quantize_block32(o, lane, a.oq + row + (size_t)blk * 32, a.od + (size_t)b * nblk + blk,
-                     a.os16 + ((size_t)b * nblk + blk) * 2);
-  }
-}
-
 constexpr int kStages = 8;   // pages in flight per CTA (two per warp)
 
 // One CTA = (split, kv head, sequence).  Warp w owns pages w, w+4, w+8, ... of the CTA's range and
@@ -295,19 +280,30 @@ __global__ void __launch_bounds__(128) attn_decode_kernel(const __grid_constant_
     __syncthreads();
     if (!s_last) return;
     __threadfence();
-    // The partial results of all splits: a warp per head finds the maximum and the sum, a lane per split, then each
-    // thread adds up its dim with the loads of four splits and all heads in flight.  One split after another, each load waits for
-    // the last: 5 splits of 4 heads took 10 of the 16.5 us of one sequence of 2048 tokens, and more splits took longer.
+    // The partial results of all splits, in two trips to L2: a warp per head takes the maxima and sums, two splits a lane, and turns them into
+    // factors; then each thread adds up its dim with the loads of four splits and all heads in flight.  One split after another,
+    // each load waits for the last: 5 splits of 4 heads took 10 of the 16.5 us of one sequence of 2048 tokens.
     const size_t p0 = ((size_t)b * a.Hkv + kh) * a.S * G;
+    const float* ml = a.part_ml + p0 * 2;
+    auto partial = [&](size_t i) { return make_float2(__ldcg(ml + 2 * i), __ldcg(ml + 2 * i + 1)); };
     float* factor = &s_acc[0][0][0];               // [splits of a chunk][G]; its last readers are behind the barriers above
     constexpr int CHUNK = 4 * DV;
+    static_assert(CHUNK >= 64, "a lane's first two splits lie in the first chunk");
     for (int g = warp; g < G; g += 4) {
-      float M = -INFINITY, L = 0.f;
-      for (int s = lane; s < a.S; s += 32) M = fmaxf(M, __ldcg(a.part_ml + (p0 + (size_t)s * G + g) * 2));
+      const float2 none = make_float2(-INFINITY, 0.f);
+      const float2 v0 = lane < a.S ? partial(lane * G + g) : none, v1 = lane + 32 < a.S ? partial((lane + 32) * G + g) : none;
+      float M = fmaxf(v0.x, v1.x);
+      for (int s = lane + 64; s < a.S; s += 32) M = fmaxf(M, partial((size_t)s * G + g).x);
       M = warp_max(M);
-      for (int s = lane; s < a.S; s += 32) {
-        const float* ml = a.part_ml + (p0 + (size_t)s * G + g) * 2;
-        L += __ldcg(ml + 1) * exp_scale(__ldcg(ml), M);
+      const float f0 = exp_scale(v0.x, M), f1 = exp_scale(v1.x, M);
+      float L = v0.y * f0 + v1.y * f1;
+      if (lane < a.S) factor[lane * G + g] = f0;
+      if (lane + 32 < a.S) factor[(lane + 32) * G + g] = f1;
+      for (int s = lane + 64; s < a.S; s += 32) {
+        const float2 v = partial((size_t)s * G + g);
+        const float f = exp_scale(v.x, M);
+        L += v.y * f;
+        if (s < CHUNK) factor[s * G + g] = f;
       }
       L = warp_sum(L);
       if (lane == 0) {
@@ -321,8 +317,10 @@ __global__ void __launch_bounds__(128) attn_decode_kernel(const __grid_constant_
     for (int s0 = 0; s0 < a.S; s0 += CHUNK) {
       const int n = min(CHUNK, a.S - s0);
       __syncthreads();
-      for (int i = tid; i < n * G; i += 128) factor[i] = exp_scale(__ldcg(a.part_ml + (p0 + (size_t)s0 * G + i) * 2), s_ml[0][i % G][0]);
-      __syncthreads();
+      if (s0) {
+        for (int i = tid; i < n * G; i += 128) factor[i] = exp_scale(partial((size_t)s0 * G + i).x, s_ml[0][i % G][0]);
+        __syncthreads();
+      }
       if (e < DV) {
         const float* src = a.part_acc + (p0 + (size_t)s0 * G) * DV + e;
 #pragma unroll 4
@@ -341,20 +339,44 @@ __global__ void __launch_bounds__(128) attn_decode_kernel(const __grid_constant_
   }
 
   if (warp * 32 < DV) {  // warps that own real output dims (all four when DV = 128)
+    // Each option is asked for once, around the loop over the heads, whose loads and arithmetic are then in flight together.
+    float o[GT];
+    if (a.sinks) {
 #pragma unroll
-    for (int g = 0; g < GT; g++) {
-      if (g >= G) continue;
-      float M = fm[g], L = fl[g], A = fa[g];
-      if (a.sinks) {
-        const float sk = a.sinks[kh * G + g];
-        const float M2 = fmaxf(M, sk);
-        const float c = exp_scale(M, M2);
-        L = L * c + __expf(sk - M2);
-        A *= c;
+      for (int g = 0; g < GT; g++) {
+        if (g >= G) continue;
+        const float sk = a.sinks[kh * G + g], M2 = fmaxf(fm[g], sk), c = exp_scale(fm[g], M2);
+        fl[g] = fl[g] * c + __expf(sk - M2);
+        fa[g] *= c;
       }
-      float o = L > 0.f ? A / L : 0.f;
-      if (a.gate) o *= 1.f / (1.f + __expf(-a.gate[(size_t)b * a.ldg + kh * G + g]));
-      write_out<DV>(a, b, kh * G + g, e, o);
+    }
+#pragma unroll
+    for (int g = 0; g < GT; g++)
+      if (g < G) o[g] = fl[g] > 0.f ? fa[g] / fl[g] : 0.f;
+    if (a.gate) {
+#pragma unroll
+      for (int g = 0; g < GT; g++)
+        if (g < G) o[g] *= 1.f / (1.f + __expf(-a.gate[(size_t)b * a.ldg + kh * G + g]));
+    }
+    const size_t row = (size_t)b * a.Hq * DV;
+    if (a.out_f32) {
+#pragma unroll
+      for (int g = 0; g < GT; g++)
+        if (g < G) a.out_f32[row + (kh * G + g) * DV + e] = o[g];
+    }
+    if (a.out_bf16) {
+#pragma unroll
+      for (int g = 0; g < GT; g++)
+        if (g < G) a.out_bf16[row + (kh * G + g) * DV + e] = __float2bfloat16(o[g]);
+    }
+    if (a.oq) {
+      const size_t nblk = (size_t)a.Hq * DV / 32;
+#pragma unroll
+      for (int g = 0; g < GT; g++) {
+        if (g >= G) continue;
+        const int blk = ((kh * G + g) * DV + e) >> 5;
+        quantize_block32(o[g], lane, a.oq + row + (size_t)blk * 32, a.od + (size_t)b * nblk + blk, a.os16 + ((size_t)b * nblk + blk) * 2);
+      }
     }
   }
 }

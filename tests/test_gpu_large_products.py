@@ -393,3 +393,27 @@ def test_few_row_products_with_weights_loaded_ahead(M, K, N, add):
     tol = _bound(A, B) + 1e-5
     assert ((outs[0] - outs[1]).abs() <= 2 * tol).all()
     assert ((outs[0] - A.float() @ B.float().t() - (x0 if add else 0)).abs() <= tol).all() and int(status) == 0
+
+
+@pytest.mark.parametrize("hd,Hq,Hkv", [(64, 8, 2), (128, 4, 4), (64, 6, 2), (128, 16, 1)])
+@pytest.mark.parametrize("S", [1, 2, 31, 33, 65, 300])             # splits of one lane's first and second, of more than 64, and of more than one chunk of factors
+@pytest.mark.parametrize("use_sinks", [False, True])
+def test_decode_attention_merges_any_number_of_splits(hd, Hq, Hkv, S, use_sinks):
+    """Splits without a page among them, and every form of the output."""
+    from test_gpu_kernels import _paged_kv
+
+    from openagents_b200.oracle import nn
+    ops, lens = _ops(), [1, 700, 333]
+    kc, vc, table, Ks, Vs = _paged_kv(3, Hkv, hd, lens, seed=80)
+    q = _randn(3, Hq * hd, seed=81) * (2.0 / hd ** 0.5)
+    sinks = _randn(Hq, seed=82) if use_sinks else None
+    scratch, counters = torch.full((ops.attn_decode_scratch_floats(3, Hq, Hkv, hd, S) + 1,), float("nan"), device=DEV), torch.zeros(3 * Hq, dtype=torch.int32, device=DEV)
+    out, outb, status = torch.empty((3, Hq * hd), device=DEV), torch.empty((3, Hq * hd), dtype=torch.bfloat16, device=DEV), torch.zeros(1, dtype=torch.int32, device=DEV)
+    for _ in range(2):                                             # the counters are left as they were
+        ops.attn_decode(q, kc, vc, table, torch.tensor(lens, dtype=torch.int32, device=DEV), 3, Hq, Hkv, hd, S=S, sinks=sinks, out_f32=out, out_bf16=outb,
+                        scratch=scratch[1:], counters=counters, status=status)       # scratch that starts on four bytes only
+        for b in range(3):
+            ref = nn.attention(q[b:b + 1].cpu().view(1, Hq, hd), Ks[b], Vs[b], torch.tensor([lens[b] - 1]), torch.arange(lens[b]),
+                               sinks=sinks.cpu() if use_sinks else None, scale=1.0).reshape(-1)
+            assert torch.allclose(out[b].cpu(), ref, atol=3e-3, rtol=3e-3), (b, (out[b].cpu() - ref).abs().max())
+        assert torch.equal(outb, out.bfloat16()) and int(counters.abs().sum()) == 0 and int(status) == 0
