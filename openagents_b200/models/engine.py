@@ -257,8 +257,8 @@ class LlamaEngine(PagedEngine):
         return (self.comm.heap.table, self.slots_off, self.slot_rows, self.xpart)
 
     # ------------------------------------------------------------------ building blocks
-    def _splits(self, B: int, ctx_pages: int) -> int:
-        return self._attn_splits(B, self.Hkv, ctx_pages)
+    def _splits(self, B: int, ctx_pages: int, window: int) -> int:
+        return self._attn_splits(B, self.Hkv, min(ctx_pages, window // PAGE + 2) if window else ctx_pages)
 
     @property
     def _sig(self):
@@ -279,7 +279,6 @@ class LlamaEngine(PagedEngine):
     def _layers_small(self, nb: int, max_ctx_pages: int):
         """<= 8 tokens, one per sequence: quantized mat-vec path."""
         cfg, x = self.cfg, self.x[:nb]
-        S = self._splits(nb, max_ctx_pages)
         qd = self.Hq * self.hd
         style = 0 if cfg.rope_style == "pairs" else 1
         n = 0
@@ -302,7 +301,7 @@ class LlamaEngine(PagedEngine):
                             self.hd, PAGE, cfg.rope_theta, style, 1.0 / math.sqrt(self.hd), table=self.rope_tab)
             oq8 = L.wo.quantized
             ops.attn_decode(self.q32, self.kc[li], self.vc[li], self.page_table, self.seq_lens, nb, self.Hq, self.Hkv,
-                            self.hd, window=L.window, S=S, sinks=L.sinks, out_f32=None if oq8 else self.xf,
+                            self.hd, window=L.window, S=self._splits(nb, max_ctx_pages, L.window), sinks=L.sinks, out_f32=None if oq8 else self.xf,
                             oq=self.xq if oq8 else None, od=self.xd, os16=self.xs, scratch=self.attn_scratch,
                             counters=self.attn_counters, status=self.status)
             if self.world == 1:
@@ -363,7 +362,6 @@ class LlamaEngine(PagedEngine):
         hb_f = self.hb2[:T]                           # its own buffer: the fused gate/up GEMM reads hb_d while writing it
         qkv = self.qkv[:T]
         gu = self.gu[:T]
-        S = self._splits(n_seqs, max_ctx_pages) if decode else 1
         n = 0
         fused = T <= (FUSED_MAX_TOKENS if self.world == 1 else QGEMM_MAX_TOKENS)
         slots = self.slots_dense and fused
@@ -382,7 +380,7 @@ class LlamaEngine(PagedEngine):
                 ops.rope_kv(qkv, self.pos, self.slot, self.q32, None, self.kc[li], self.vc[li], self.Hq, self.Hkv, self.hd,
                             PAGE, cfg.rope_theta, style, 1.0 / math.sqrt(self.hd), table=self.rope_tab)
                 ops.attn_decode(self.q32, self.kc[li], self.vc[li], self.page_table, self.seq_lens, n_seqs, self.Hq,
-                                self.Hkv, self.hd, window=L.window, S=S, sinks=L.sinks, out_bf16=hb_q,
+                                self.Hkv, self.hd, window=L.window, S=self._splits(n_seqs, max_ctx_pages, L.window), sinks=L.sinks, out_bf16=hb_q,
                                 scratch=self.attn_scratch, counters=self.attn_counters, status=self.status)
             else:
                 ops.rope_kv(qkv, self.pos, self.slot, None, self.q16, self.kc[li], self.vc[li], self.Hq, self.Hkv, self.hd,

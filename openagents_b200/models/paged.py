@@ -235,15 +235,22 @@ class PagedEngine:
         return bad
 
     def _attn_splits(self, B: int, kv_heads: int, ctx_pages: int) -> int:
-        """Split-K factor of decode attention.  Measured on the 8B shape: small batches want two CTAs per SM of at least
-        16 pages (1 x 2048 tokens: 5 splits 2.31 ms a step, 8 splits 2.29, 24 splits 2.31; 7 x 1500: 3 splits 3.32, 6
-        splits 3.21, 12 splits 3.39), large batches run best at ~2000 CTAs (several waves even out the tail) of at
-        least 32 pages (32 x 1000: 1 split 3.52, 2 splits 3.78)."""
+        """Split-K factor of decode attention over ``ctx_pages`` pages (a window's, where a layer has one).  The merge of the partial results costs some
+        3 us, as much as 15 pages: one split below 48.  Then up to two or three CTAs per SM of at least 10 pages; with a row per
+        SM and more, some 2000 CTAs (several waves even out the tail) of at least 32 pages, or 24 while two splits fit in one wave.  Measured,
+        us, splits: time (32 query heads on 8 of size 128): 1 x 512 tokens 1: 8.7, 2: 8.2, 8: 6.4, but of size 64 1: 6.9, 2: 9.4; 1 x 2048 1: 26.9,
+        5: 10.5, 12: 8.7; 7 x 2048 1: 27.3, 3: 17.8, 6: 14.1, 12: 17.5; 20 x 1000 1: 20.7, 2: 16.4; 32 x 1000 1: 25.7, 2: 34.1 (a second
+        wave nearly empty), 3: 30.8; 64 x 2048 1: 101, 4: 90."""
         if self.attn_target_ctas:                      # explicit override (benchmark sweeps)
             want = max(1, (self.attn_target_ctas + B * kv_heads - 1) // (B * kv_heads))
         else:
             rows = B * kv_heads
-            want = min(ctx_pages // 16, (296 + rows - 1) // rows) if rows < 148 else min(ctx_pages // 32, (2048 + rows - 1) // rows)
+            if rows < 148:
+                want = min(16, ctx_pages // 10, (370 + rows - 1) // rows) if ctx_pages >= 48 else 1
+            else:
+                want = min(ctx_pages // (24 if rows <= 222 else 32), (2048 + rows - 1) // rows)
+                if want == 2 and 222 < rows < 444:
+                    want = 3
         return max(1, min(self.max_splits, want, ctx_pages))
 
     # ------------------------------------------------------------------ host-side batch assembly
