@@ -385,7 +385,7 @@ class LlamaEngine(PagedEngine):
             else:
                 ops.rope_kv(qkv, self.pos, self.slot, None, self.q16, self.kc[li], self.vc[li], self.Hq, self.Hkv, self.hd,
                             PAGE, cfg.rope_theta, style, 1.0 / math.sqrt(self.hd), table=self.rope_tab)
-                if self._tc05_prefill(L):     # 5th-generation tensor-core path
+                if self._tc05_prefill(L, n_seqs, max_q, max_ctx_pages * PAGE):     # 5th-generation tensor-core path
                     ops.attn_prefill_tc05(self.q16, self.kc[li], self.vc[li], self.page_table, self.q_start, self.q_len,
                                           self.seq_lens, n_seqs, max_q, self.Hq, self.Hkv, window=L.window, sinks=L.sinks,
                                           out_bf16=hb_q, status=self.status, dk=self.hd, dv=self.hd)
@@ -405,10 +405,16 @@ class LlamaEngine(PagedEngine):
             self._slots_pending = slots      # decode: the final norm takes the last sum
         return n
 
-    def _tc05_prefill(self, L: _Layer) -> bool:
-        """Whether a layer's prefill attention runs on tcgen05 rather than mma.sync.  Head size 64: 4096 tokens of 64 heads take 337 us
-        against 624, but with a window of 128 (three key blocks per query block, little to pipeline) 112 against 76."""
-        return self.prefill_tc05 and (self.hd == 128 or (self.hd == 64 and not 0 < L.window < 1024))
+    def _tc05_prefill(self, L: _Layer, n_seqs: int, max_q: int, keys: int) -> bool:
+        """Whether a layer's prefill attention runs on tcgen05 rather than mma.sync, for the longest of the call's chunks and contexts.  Head size 128
+        always.  Head size 64 where there are keys enough to pipeline: its blocks of 128 queries take a whole SM, those of mma.sync
+        64 queries of a quarter.  Measured (us, tcgen05 / mma.sync): 64 heads, 1 prompt of 128 tokens 6.7 / 5.5, 320 tokens 14.6 / 12.2, 512 tokens
+        19 / 23, 4096 tokens 337 / 624; 4 prompts of 512 60 / 55, of 1024 150 / 174; 8 heads, 1 prompt of 300 8.4 / 9.2; 64 new
+        tokens behind 2000 26 / 44; a window of 128 over 4096 tokens (three key blocks per query block) 112 / 76."""
+        if not self.prefill_tc05 or self.hd != 64:
+            return self.prefill_tc05 and self.hd == 128
+        blocks = n_seqs * self.Hq * ((max_q + 127) // 128)
+        return not 0 < L.window < 1024 and (keys >= 900 or (keys >= 448 and blocks <= 3 * 148) or (keys > 256 and blocks <= 148))
 
     @nvtx_method("tp.row_parallel(all_reduce)")
     def _row_parallel(self, a_bf16, w: QWeight, T: int, x, bias, fused: bool, slots: bool, table):
@@ -459,7 +465,7 @@ class LlamaEngine(PagedEngine):
                           status=self.status, sym=table, ag_rows_per_rank=Tr, ag_epoch=self._ag_epoch)
             ops.rope_kv(qkv, self.pos, self.slot, None, self.q16, self.kc[li], self.vc[li], self.Hq, self.Hkv, self.hd,
                         PAGE, cfg.rope_theta, style, 1.0 / math.sqrt(self.hd), table=self.rope_tab)
-            if self._tc05_prefill(L):
+            if self._tc05_prefill(L, n_seqs, max_q, max_q):
                 ops.attn_prefill_tc05(self.q16, self.kc[li], self.vc[li], self.page_table, self.q_start, self.q_len,
                                       self.seq_lens, n_seqs, max_q, self.Hq, self.Hkv, window=L.window, sinks=L.sinks,
                                       out_bf16=hb_q, status=self.status, dk=self.hd, dv=self.hd)

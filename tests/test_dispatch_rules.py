@@ -38,3 +38,23 @@ def test_attention_splits_follow_a_layers_window():
     assert LlamaEngine._splits(eng, 1, 256, 0) > 8                 # a long context is split
     assert LlamaEngine._splits(eng, 1, 256, 128) == 1              # ten pages of it are not
     assert LlamaEngine._splits(eng, 1, 20, 4096) == LlamaEngine._splits(eng, 1, 20, 0)
+
+
+# us on tcgen05 and on mma.sync, head size 64: (query heads, prompts, tokens of each, tokens ahead of them)
+PROMPTS_64 = {
+    (64, 1, 40, 0): (5.9, 4.1), (64, 1, 128, 0): (6.7, 5.5), (64, 1, 320, 0): (14.6, 12.2), (64, 1, 512, 0): (19.0, 22.7), (64, 1, 1200, 0): (58.4, 76.6),
+    (64, 4, 256, 0): (27.6, 21.5), (64, 4, 512, 0): (60.2, 55.4), (64, 4, 1024, 0): (150.0, 174.0), (8, 1, 300, 0): (8.4, 9.2), (8, 1, 100, 0): (6.1, 5.2),
+    (8, 4, 512, 0): (10.4, 16.2), (64, 1, 16, 2000): (23.3, 42.8), (64, 4, 64, 2000): (51.7, 56.5), (64, 8, 128, 0): (24.7, 14.1),
+}
+
+
+def test_prefill_attention_of_head_size_64_takes_the_faster_kernel():
+    from openagents_b200.models.engine import LlamaEngine
+    layer = lambda window: types.SimpleNamespace(window=window)
+    for (heads, prompts, tokens, past), (tc05, mma) in PROMPTS_64.items():
+        eng = types.SimpleNamespace(hd=64, Hq=heads, prefill_tc05=True)
+        assert LlamaEngine._tc05_prefill(eng, layer(0), prompts, tokens, tokens + past) == (tc05 < mma), (heads, prompts, tokens, past)
+        assert not LlamaEngine._tc05_prefill(eng, layer(128), prompts, tokens, tokens + past)
+    assert LlamaEngine._tc05_prefill(types.SimpleNamespace(hd=128, Hq=32, prefill_tc05=True), layer(0), 1, 1, 1)
+    assert not LlamaEngine._tc05_prefill(types.SimpleNamespace(hd=128, Hq=32, prefill_tc05=False), layer(0), 1, 4096, 4096)
+    assert not LlamaEngine._tc05_prefill(types.SimpleNamespace(hd=256, Hq=32, prefill_tc05=True), layer(0), 1, 4096, 4096)
