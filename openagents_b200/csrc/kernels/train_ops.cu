@@ -138,8 +138,8 @@ B200_API int b200_layernorm_fwd(const void* x, const float* g, const float* b, f
 // dx = rstd * (dy*g - mean(dy*g) - xhat * mean(dy*g*xhat)); dgamma += dy*xhat; dbeta += dy.
 // Each CTA walks rows with a grid stride, keeps its gamma/beta partial sums in shared memory and
 // adds them to the fp32 gradients once at the end.  `dx_add`: accumulate into dx (residual branch).
-// NJ: 256-column steps of a row that stays in registers (D <= NJ * 256; 0: rows of any length, read twice).  As many as D needs: with
-// room for 1024 columns whatever D, 158 registers left one CTA per SM, and 16384 rows of 768 (100 MB) took 47 us, now 35.
+// NJ: 256-column steps of a row that stays in registers (D <= NJ * 256; 0: rows of any length, read twice).  As many as D needs: room for
+// 1024 columns takes 158 registers, which leaves one CTA per SM.
 template <int NJ>
 __global__ void __launch_bounds__(256, NJ == 4 ? 1 : 2)
     layernorm_bwd_kernel(const bf16* __restrict__ dy, const bf16* __restrict__ x,
@@ -271,7 +271,10 @@ B200_API int b200_layernorm_bwd(const void* dy, const void* x, const float* g, c
   if (D % 8) return B200_ERR_BAD_ARG;
   auto kern = D <= 256 ? layernorm_bwd_kernel<1> : D <= 512 ? layernorm_bwd_kernel<2> : D <= 768 ? layernorm_bwd_kernel<3>
               : D <= 1024 ? layernorm_bwd_kernel<4> : layernorm_bwd_kernel<0>;
-  const int grid = min((rows + 7) / 8, D > 768 && D <= 1024 ? 148 : 296);      // what is resident at once
+  // One CTA per SM, or two.  A CTA ends by adding its 2 D column sums into the gradients, so two pay only where the walk over the rows is long
+  // beside that (rows of 768, us with 148 / 296 CTAs: 2048 rows 10.8 / 15.3, 10240 rows 21.5 / 21.9, 16384 rows 29.0 / 26.8) or the
+  // rows are read twice (2048 rows of 1600: 26.9 / 16.8).  A row of up to 1024 values in registers leaves room for one.
+  const int grid = min((rows + 7) / 8, D > 1024 || (D <= 768 && rows >= 12288) ? 296 : 148);
   kern<<<grid, 256, 2 * D * sizeof(float), st>>>((const bf16*)dy, (const bf16*)x, g, mean, rstd, (bf16*)dx, dx_add, dgamma, dbeta, rows, D);
   return (int)cudaGetLastError();
 }

@@ -417,3 +417,19 @@ def test_decode_attention_merges_any_number_of_splits(hd, Hq, Hkv, S, use_sinks)
                                sinks=sinks.cpu() if use_sinks else None, scale=1.0).reshape(-1)
             assert torch.allclose(out[b].cpu(), ref, atol=3e-3, rtol=3e-3), (b, (out[b].cpu() - ref).abs().max())
         assert torch.equal(outb, out.bfloat16()) and int(counters.abs().sum()) == 0 and int(status) == 0
+
+
+@pytest.mark.parametrize("rows,D", [(12287, 768), (12288, 768), (12288, 64), (2400, 1024), (2400, 1032)])      # either side of where two CTAs an SM take over
+def test_layernorm_backward_grids(rows, D):
+    from openagents_b200.ops import train_ops as tops
+    x, dy = _randn(rows, D, seed=83).bfloat16(), _randn(rows, D, seed=84).bfloat16()
+    g, b = _randn(D, seed=85), _randn(D, seed=86)
+    y, mean, rstd = torch.empty_like(x), torch.empty(rows, device=DEV), torch.empty(rows, device=DEV)
+    tops.layernorm_fwd(x, g, b, 1e-5, y, mean, rstd)
+    dx, dg, db = torch.zeros_like(x), torch.zeros(D, device=DEV), torch.zeros(D, device=DEV)
+    tops.layernorm_bwd(dy, x, g, mean, rstd, dx, False, dg, db)
+    xr, gr, br = (t.double().requires_grad_(True) for t in (x, g, b))
+    torch.nn.functional.layer_norm(xr, (D,), gr, br, 1e-5).backward(dy.double())
+    assert ((dx.double() - xr.grad).abs() <= 2.0 ** -8 * xr.grad.abs() + 1e-4).all()
+    for got, ref in ((dg, gr.grad), (db, br.grad)):
+        assert ((got.double() - ref).abs() <= 2.0 ** -18 * rows + 1e-4).all()
