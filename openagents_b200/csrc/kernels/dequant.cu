@@ -7,21 +7,20 @@ using namespace b200;
 
 enum { WT_Q4KR = 0, WT_Q6KR = 1, WT_Q8R = 2, WT_BF16 = 3, WT_MXFP4R = 4 };
 
-// Q4_K-R and Q6_K-R.  Rows are whole superblocks, so the matrix is one run of them and needs no division; a warp expands kPerWarp
+// Q4_K-R and Q6_K-R.  Rows are whole superblocks, so the matrix is one run of them and needs no division; a warp expands PER
 // superblocks, a lane one word (8 elements) of each, all loads ahead of the arithmetic.  It runs beside the GEMM on the matrix before
 // (prefill), so that its instructions count as much as its bytes.  With a 64-bit division and integer conversions per word it took
 // 46 us for an average matrix of an 8B layer (140 MB).
-constexpr int kPerWarp = 4;
-template <int WT>
+template <int WT, int PER>
 __global__ void __launch_bounds__(256) dequant_superblocks_kernel(const uint8_t* __restrict__ w, const __half* __restrict__ d6,
                                                                   __nv_bfloat16* __restrict__ out, size_t n_sb) {
   constexpr int BYTES = WT == WT_Q4KR ? 144 : 208;
   const int lane = threadIdx.x & 31;
-  const size_t first = ((size_t)blockIdx.x * 8 + (threadIdx.x >> 5)) * kPerWarp;
-  uint4 hdr[kPerWarp];
-  uint32_t q[kPerWarp];
+  const size_t first = ((size_t)blockIdx.x * 8 + (threadIdx.x >> 5)) * PER;
+  uint4 hdr[PER];
+  uint32_t q[PER];
 #pragma unroll
-  for (int i = 0; i < kPerWarp; i++) {
+  for (int i = 0; i < PER; i++) {
     const uint8_t* blk = w + min(first + i, n_sb - 1) * BYTES;
     if constexpr (WT == WT_Q4KR) {
       hdr[i] = __ldg((const uint4*)blk);
@@ -34,7 +33,7 @@ __global__ void __launch_bounds__(256) dequant_superblocks_kernel(const uint8_t*
     }
   }
 #pragma unroll
-  for (int i = 0; i < kPerWarp; i++) {
+  for (int i = 0; i < PER; i++) {
     if (first + i >= n_sb) return;
     uint32_t o[4];
     if constexpr (WT == WT_Q4KR) {
@@ -73,6 +72,15 @@ __global__ void __launch_bounds__(256) dequant_superblocks_kernel(const uint8_t*
   }
 }
 
+template <int WT>
+static int launch_superblocks(const uint8_t* w, const __half* d6, __nv_bfloat16* out, size_t n_sb, cudaStream_t st) {
+  // Four superblocks a warp once that still fills the SMs (us with one / four, Q6_K: 512 x 512 1.9 / 2.8, 2048 x 2048 4.1 / 4.5,
+  // 4096 x 2048 6.5 / 6.1).
+  if (n_sb < 16384) dequant_superblocks_kernel<WT, 1><<<(unsigned)((n_sb + 7) / 8), 256, 0, st>>>(w, d6, out, n_sb);
+  else dequant_superblocks_kernel<WT, 4><<<(unsigned)((n_sb + 31) / 32), 256, 0, st>>>(w, d6, out, n_sb);
+  return (int)cudaGetLastError();
+}
+
 // Q8_0-R and MXFP4-R: one thread expands one 8-element word.
 __global__ void dequant_kernel(int wt, const uint8_t* __restrict__ w, const uint8_t* __restrict__ w2,
                                __nv_bfloat16* __restrict__ out, size_t n_words) {
@@ -107,15 +115,8 @@ B200_API int b200_dequant_bf16(int wt, const void* w, const void* w2, void* out,
   if (K % 32) return B200_ERR_BAD_ARG;
   if ((wt == WT_Q4KR || wt == WT_Q6KR) && K % 256) return B200_ERR_BAD_ARG;
   const size_t n_words = N * (size_t)K / 8, n_sb = N * (size_t)K / 256;
-  const unsigned blocks = (unsigned)((n_sb + 8 * kPerWarp - 1) / (8 * kPerWarp));
-  if (wt == WT_Q4KR) {
-    dequant_superblocks_kernel<WT_Q4KR><<<blocks, 256, 0, st>>>((const uint8_t*)w, nullptr, (__nv_bfloat16*)out, n_sb);
-    return (int)cudaGetLastError();
-  }
-  if (wt == WT_Q6KR) {
-    dequant_superblocks_kernel<WT_Q6KR><<<blocks, 256, 0, st>>>((const uint8_t*)w, (const __half*)w2, (__nv_bfloat16*)out, n_sb);
-    return (int)cudaGetLastError();
-  }
+  if (wt == WT_Q4KR) return launch_superblocks<WT_Q4KR>((const uint8_t*)w, nullptr, (__nv_bfloat16*)out, n_sb, st);
+  if (wt == WT_Q6KR) return launch_superblocks<WT_Q6KR>((const uint8_t*)w, (const __half*)w2, (__nv_bfloat16*)out, n_sb, st);
   dequant_kernel<<<(unsigned)((n_words + 255) / 256), 256, 0, st>>>(wt, (const uint8_t*)w, (const uint8_t*)w2,
                                                                      (__nv_bfloat16*)out, n_words);
   return (int)cudaGetLastError();

@@ -433,3 +433,18 @@ def test_layernorm_backward_grids(rows, D):
     assert ((dx.double() - xr.grad).abs() <= 2.0 ** -8 * xr.grad.abs() + 1e-4).all()
     for got, ref in ((dg, gr.grad), (db, br.grad)):
         assert ((got.double() - ref).abs() <= 2.0 ** -18 * rows + 1e-4).all()
+
+
+@pytest.mark.parametrize("kind", ["Q4_K", "Q6_K"])
+@pytest.mark.parametrize("N,K", [(1, 256), (3, 1280), (5461, 768), (16384, 256), (4100, 1024)])      # 1, 15, 16383, 16384 and 16400 superblocks
+def test_expansion_of_any_number_of_superblocks(kind, N, K):
+    from openagents_b200.gguf import GgmlType
+    from openagents_b200.gguf import torch_codecs as tc
+    from openagents_b200.models.qweight import QWeight, RawTensor
+    t = GgmlType[kind]
+    raw = tc.quantize(_randn(N, K, seed=87), t)
+    out = torch.full((N + 1, K), 7.0, dtype=torch.bfloat16, device=DEV)
+    QWeight.from_raw(RawTensor(t, (N, K), raw)).dequant_into(out[:N])
+    want = tc.dequantize(raw, t, (N, K))
+    # one rounding to bf16, of a multiply-add in 32 bits whose terms are of the block's size
+    assert ((out[:N].float() - want).abs() <= 2.0 ** -8 * want.abs() + 2.0 ** -20 * want.abs().max()).all() and (out[N] == 7.0).all()
