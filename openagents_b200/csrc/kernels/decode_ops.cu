@@ -207,7 +207,7 @@ __global__ void __launch_bounds__(1024) rmsnorm_kernel(float* __restrict__ x, co
 
 // Many rows (prefill): what bounds the kernel above there is not memory but its own chain of load, two block-wide barriers and store,
 // with two 1024-thread blocks on an SM: 44 us for 2048 rows of 4096, 50 MB.  Here a row takes 256 threads with 16-byte loads, eight
-// rows are in flight per SM and 11 us remain.
+// rows are in flight per SM and 10 us remain.
 constexpr int kRowThreads = 256, kRowVecs = 8;       // rows of up to 4 * 256 * 8 values
 __global__ void __launch_bounds__(kRowThreads) rmsnorm_rows_kernel(const float4* __restrict__ x, const float4* __restrict__ g, float eps, int D,
                                                                    uint2* __restrict__ hb, float4* __restrict__ hf) {
@@ -251,8 +251,9 @@ B200_API int b200_rmsnorm(float* x, const float* g, float eps, int T, int D, voi
                           size_t slot_off, int slot_rows, float* part, cudaStream_t st) {
   if (D % 32 || (zero && ((zero_n % 4) || ((uintptr_t)zero % 16)))) return B200_ERR_BAD_ARG;
   if ((sym_mode != 0 && !sym) || sym_mode < 0 || sym_mode > 2 || (sym_mode == 2 && (T > slot_rows || slot_rows > kSymSlotRows || (slot_off % 16) || !part || (D % 4) || ((uintptr_t)part % 16)))) return B200_ERR_BAD_ARG;
-  // From 128 rows on (as many as make a block per SM) rows in flight count for more than the latency of one.
-  if (T >= 128 && sym_mode == 0 && !xq && !zero && D <= 4 * kRowThreads * kRowVecs &&
+  // From 128 rows on rows in flight count for more than the latency of one; rows of more than 4096 values wait until there are more of
+  // them than SMs (144 rows of 8192, both outputs: 4.2 us against 4.0; 160 rows 4.5 against 6.7).
+  if (T >= (D <= 4096 ? 128 : 149) && sym_mode == 0 && !xq && !zero && D <= 4 * kRowThreads * kRowVecs &&
       !(((uintptr_t)x | (uintptr_t)g | (uintptr_t)hf) & 15) && !((uintptr_t)hb & 7))
     return launch_pdl(rmsnorm_rows_kernel, dim3(T), dim3(kRowThreads), 0, st, (const float4*)x, (const float4*)g, eps, D, (uint2*)hb, (float4*)hf);
   const int threads = D >= 4096 ? 1024 : D >= 1024 ? 512 : 256;
@@ -506,8 +507,9 @@ B200_API int b200_rope_kv(const float* qkv, const int* pos, const int* slot, flo
                           void* vc, int T, int Hq, int Hkv, int hd, int page_size, float theta,
                           int style, float q_scale, const void* tab, int tab_len, cudaStream_t st) {
   if (hd % 2) return B200_ERR_BAD_ARG;
-  // As for the norm: from 128 tokens on the wide accesses win, below it the many small blocks finish sooner.
-  if (T >= 128 && hd % (style == 0 ? 8 : 16) == 0 &&
+  // From 128 tokens and 256 K values on the wide accesses win; below it the many small blocks finish sooner (us, halves rotated, old / new:
+  // 128 x 15 heads of 64 2.0 / 2.6, 256 x 15 2.6 / 2.6, 128 x 36 heads 2.6 / 2.5, 128 x 48 heads of 128 3.7 / 3.5).
+  if (T >= 128 && (long)T * (Hq + 2 * Hkv) * hd >= 1 << 18 && hd % (style == 0 ? 8 : 16) == 0 &&
       !(((uintptr_t)qkv | (uintptr_t)q_out | (uintptr_t)q_out_h | (uintptr_t)kc | (uintptr_t)vc) & 15))
     return launch_pdl(style == 0 ? rope_kv_rows_kernel<0> : rope_kv_rows_kernel<1>, dim3(T), dim3(256), 0, st, qkv, pos, slot, q_out, (__half*)q_out_h,
                       (__half*)kc, (__half*)vc, Hq, Hkv, hd, page_size, theta, q_scale, (const float2*)tab, tab_len);

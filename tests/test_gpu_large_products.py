@@ -448,3 +448,32 @@ def test_expansion_of_any_number_of_superblocks(kind, N, K):
     want = tc.dequantize(raw, t, (N, K))
     # one rounding to bf16, of a multiply-add in 32 bits whose terms are of the block's size
     assert ((out[:N].float() - want).abs() <= 2.0 ** -8 * want.abs() + 2.0 ** -20 * want.abs().max()).all() and (out[N] == 7.0).all()
+
+
+@pytest.mark.parametrize("T,Hq,Hkv", [(128, 16, 8), (128, 15, 8), (146, 13, 7), (147, 13, 7), (127, 64, 8)])      # 2^18 values, below and above; 128 tokens
+@pytest.mark.parametrize("style", ["pairs", "half"])
+def test_rope_kv_either_side_of_the_wide_kernel(T, Hq, Hkv, style):
+    """Against the same tokens a few at a time."""
+    ops, hd, st = _ops(), 64, 0 if style == "pairs" else 1
+    qkv, pos = _randn(T, (Hq + 2 * Hkv) * hd, seed=88), torch.arange(T, device=DEV).int()
+    tab = ops.rope_table(256, hd, 10000.0, DEV)
+    outs = []
+    for step in (T, 50):
+        kc = torch.zeros((T // 16 + 1, Hkv, 16, hd), dtype=torch.float16, device=DEV)
+        vc, q16 = torch.zeros_like(kc), torch.empty((T, Hq * hd), dtype=torch.float16, device=DEV)
+        for lo in range(0, T, step):
+            s = slice(lo, lo + step)
+            ops.rope_kv(qkv[s], pos[s], pos[s], None, q16[s], kc, vc, Hq, Hkv, hd, 16, 10000.0, st, 0.125, table=tab)
+        outs.append((q16, kc, vc))
+    for a, b in zip(*outs):                                        # a contracted multiply-add may round differently
+        assert torch.allclose(a.float(), b.float(), rtol=2.0 ** -10, atol=1e-6)
+
+
+@pytest.mark.parametrize("T,D", [(148, 8192), (149, 8192), (148, 4128), (149, 4128), (128, 4096), (127, 4096)])
+def test_rmsnorm_either_side_of_the_many_row_kernel(T, D):
+    ops = _ops()
+    x, g = _randn(T, D, seed=89), _randn(D, seed=90)
+    hf, hb = torch.empty((T, D), device=DEV), torch.empty((T, D), dtype=torch.bfloat16, device=DEV)
+    ops.rmsnorm(x, g, 1e-5, hb=hb, hf=hf)
+    ref = x.double() * torch.rsqrt(x.double().pow(2).mean(-1, keepdim=True) + 1e-5) * g.double()
+    assert ((hf - ref).abs() <= 2.0 ** -20 * ref.abs() + 1e-12).all() and torch.equal(hb, hf.bfloat16())
