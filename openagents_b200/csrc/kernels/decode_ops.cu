@@ -206,7 +206,7 @@ __global__ void __launch_bounds__(1024) rmsnorm_kernel(float* __restrict__ x, co
 }
 
 // Many rows (prefill): what bounds the kernel above there is not memory but its own chain of load, two block-wide barriers and store,
-// with two 1024-thread blocks on an SM: 44 us for 2048 rows of 4096, 50 MB.  Here a row takes 256 threads with 16-byte loads, eight
+// with two 1024-thread blocks on an SM: 49 us for 2048 rows of 4096, 50 MB.  Here a row takes 256 threads with 16-byte loads, eight
 // rows are in flight per SM and 10 us remain.
 constexpr int kRowThreads = 256, kRowVecs = 8;       // rows of up to 4 * 256 * 8 values
 __global__ void __launch_bounds__(kRowThreads) rmsnorm_rows_kernel(const float4* __restrict__ x, const float4* __restrict__ g, float eps, int D,
@@ -402,7 +402,7 @@ __global__ void rope_kv_kernel(const float* __restrict__ qkv, const int* __restr
 }
 
 // The same for many tokens: a block takes a token and a thread eight values of a head (style 1: eight of each half) with 16-byte
-// loads and stores.  The kernel above takes 51 us for 2048 tokens of 48 heads of 128 (75 MB): its two-byte stores and
+// loads and stores.  The kernel above takes 43 us for 2048 tokens of 48 heads of 128 (75 MB), this one 21: its two-byte stores and
 // index arithmetic per pair bound it.
 __device__ __forceinline__ uint4 pack_half8(const float (&v)[8]) {
   uint4 o;

@@ -9,8 +9,8 @@ enum { WT_Q4KR = 0, WT_Q6KR = 1, WT_Q8R = 2, WT_BF16 = 3, WT_MXFP4R = 4 };
 
 // Q4_K-R and Q6_K-R.  Rows are whole superblocks, so the matrix is one run of them and needs no division; a warp expands PER
 // superblocks, a lane one word (8 elements) of each, all loads ahead of the arithmetic.  It runs beside the GEMM on the matrix before
-// (prefill), so that its instructions count as much as its bytes.  With a 64-bit division and integer conversions per word it took
-// 46 us for an average matrix of an 8B layer (140 MB).
+// (prefill), so that its instructions count as much as its bytes.  With a 64-bit division and integer conversions per word an
+// average matrix of an 8B layer (140 MB of bf16, Q4_K) takes 48 us, without them 31.
 template <int WT, int PER>
 __global__ void __launch_bounds__(256) dequant_superblocks_kernel(const uint8_t* __restrict__ w, const __half* __restrict__ d6,
                                                                   __nv_bfloat16* __restrict__ out, size_t n_sb) {

@@ -732,8 +732,8 @@ static int launch_gemm(const CUtensorMap& ta, const CUtensorMap& tb, const GemmE
 // times are estimated as waves of tiles (148 CTAs, 74 pairs) times the K blocks of a tile times the time of one, in microseconds,
 // plus what a tile's epilogue leaves uncovered.  The times per block of 64 were measured on full waves: a pair 0.36 (256 x 256) and
 // 0.21 (256 x 128), one CTA 0.43 (128 x 256), 0.33 (128 x 128) and 0.26 (128 x 64); above N = 128 they are near what the tensor
-// cores need, below it L2 bandwidth bounds them.  At M = 2048 the pairs take 305 against 335 us (N 28672, K 4096) and 76 against
-// 93 (6144); 16384 x 2304 x 768 takes 50 us against 97; 300 x 28672 x 4096 stays with single CTAs (86 against 90): 300 rows fill
+// cores need, below it L2 bandwidth bounds them.  At M = 2048 the pairs take 295 against 338 us (N 28672, K 4096) and 74 against
+// 94 (6144); 16384 x 2304 x 768 takes 51 us against 99; 300 x 28672 x 4096 stays with single CTAs (86 against 90): 300 rows fill
 // 384 of their rows but 512 of the pairs'.
 static bool choose_pair(PairGemm& g, int old_tile, int old_splits) {
   if (g.M <= 64 || !pair_takes(g)) return false;

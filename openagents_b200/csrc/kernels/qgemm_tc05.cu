@@ -324,18 +324,7 @@ __global__ void __launch_bounds__(kQThreads, 1) qgemm_kernel(const __grid_consta
           for (int k4 = 0; k4 < 8; k4++) {
             float c[4] = {__uint_as_float(v[4 * k4]) + b, __uint_as_float(v[4 * k4 + 1]) + b, __uint_as_float(v[4 * k4 + 2]) + b,
                           __uint_as_float(v[4 * k4 + 3]) + b};
-            float x0 = (lq & 1) ? c[0] : c[1];
-            x0 = __shfl_xor_sync(0xffffffffu, x0, 1);
-            if (lq & 1) c[0] = x0; else c[1] = x0;
-            float x1 = (lq & 1) ? c[2] : c[3];
-            x1 = __shfl_xor_sync(0xffffffffu, x1, 1);
-            if (lq & 1) c[2] = x1; else c[3] = x1;
-            float x2 = (lq & 2) ? c[0] : c[2];
-            x2 = __shfl_xor_sync(0xffffffffu, x2, 2);
-            if (lq & 2) c[0] = x2; else c[2] = x2;
-            float x3 = (lq & 2) ? c[1] : c[3];
-            x3 = __shfl_xor_sync(0xffffffffu, x3, 2);
-            if (lq & 2) c[1] = x3; else c[3] = x3;
+            transpose_quad(c, lq);
             const int t = t0 + 4 * k4 + lq;          // c[0..3] = columns nq .. nq + 3 of token t
             if (t >= a.T) continue;
             const size_t idx = (size_t)t * a.ldo + nq;

@@ -67,6 +67,22 @@ __device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, vo
   return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag));
 }
 
+// A 4 x 4 patch held by the four lanes of a quad, a row each (lq: the lane's place in it), transposed: four shuffles.
+__device__ __forceinline__ void transpose_quad(float (&c)[4], int lq) {
+  float x0 = (lq & 1) ? c[0] : c[1];
+  x0 = __shfl_xor_sync(0xffffffffu, x0, 1);
+  if (lq & 1) c[0] = x0; else c[1] = x0;
+  float x1 = (lq & 1) ? c[2] : c[3];
+  x1 = __shfl_xor_sync(0xffffffffu, x1, 1);
+  if (lq & 1) c[2] = x1; else c[3] = x1;
+  float x2 = (lq & 2) ? c[0] : c[2];
+  x2 = __shfl_xor_sync(0xffffffffu, x2, 2);
+  if (lq & 2) c[0] = x2; else c[2] = x2;
+  float x3 = (lq & 2) ? c[1] : c[3];
+  x3 = __shfl_xor_sync(0xffffffffu, x3, 2);
+  if (lq & 2) c[1] = x3; else c[3] = x3;
+}
+
 // Generic-proxy writes to shared memory (st.shared) must be fenced before the async proxy
 // (TMA, tcgen05.mma) reads them.
 __device__ __forceinline__ void fence_proxy_async_smem() {

@@ -164,7 +164,7 @@ __global__ void __launch_bounds__(256, NJ == 4 ? 1 : 2)
     const bf16* dr = dy + (size_t)row * D;
     const float mu = mean[row], rs = rstd[row];
     float s1 = 0.f, s2 = 0.f;
-    if (in_regs) {
+    if constexpr (in_regs) {
       uint4 kx[MAXJ], kd[MAXJ];
 #pragma unroll
       for (int j = 0; j < MAXJ; j++) {
@@ -216,34 +216,34 @@ __global__ void __launch_bounds__(256, NJ == 4 ? 1 : 2)
           *dst = pack8(o);
         }
       }
-      continue;
-    }
-    for (int i = lane * 2; i < D; i += 64) {
-      const float2 xv = __bfloat1622float2(*(const __nv_bfloat162*)(xr + i));
-      const float2 dv = __bfloat1622float2(*(const __nv_bfloat162*)(dr + i));
-      const float h0 = (xv.x - mu) * rs, h1 = (xv.y - mu) * rs;
-      const float a0 = dv.x * g[i], a1 = dv.y * g[i + 1];
-      s1 += a0 + a1;
-      s2 += a0 * h0 + a1 * h1;
-      atomicAdd(sg + i, dv.x * h0);
-      atomicAdd(sg + i + 1, dv.y * h1);
-      atomicAdd(sb + i, dv.x);
-      atomicAdd(sb + i + 1, dv.y);
-    }
-    s1 = warp_sum(s1) / D;
-    s2 = warp_sum(s2) / D;
-    for (int i = lane * 2; i < D; i += 64) {
-      const float2 xv = __bfloat1622float2(*(const __nv_bfloat162*)(xr + i));
-      const float2 dv = __bfloat1622float2(*(const __nv_bfloat162*)(dr + i));
-      const float h0 = (xv.x - mu) * rs, h1 = (xv.y - mu) * rs;
-      float o0 = rs * (dv.x * g[i] - s1 - h0 * s2), o1 = rs * (dv.y * g[i + 1] - s1 - h1 * s2);
-      __nv_bfloat162* dst = (__nv_bfloat162*)(dx + (size_t)row * D + i);
-      if (dx_add) {
-        const float2 p = __bfloat1622float2(*dst);
-        o0 += p.x;
-        o1 += p.y;
+    } else {
+      for (int i = lane * 2; i < D; i += 64) {
+        const float2 xv = __bfloat1622float2(*(const __nv_bfloat162*)(xr + i));
+        const float2 dv = __bfloat1622float2(*(const __nv_bfloat162*)(dr + i));
+        const float h0 = (xv.x - mu) * rs, h1 = (xv.y - mu) * rs;
+        const float a0 = dv.x * g[i], a1 = dv.y * g[i + 1];
+        s1 += a0 + a1;
+        s2 += a0 * h0 + a1 * h1;
+        atomicAdd(sg + i, dv.x * h0);
+        atomicAdd(sg + i + 1, dv.y * h1);
+        atomicAdd(sb + i, dv.x);
+        atomicAdd(sb + i + 1, dv.y);
       }
-      *dst = __floats2bfloat162_rn(o0, o1);
+      s1 = warp_sum(s1) / D;
+      s2 = warp_sum(s2) / D;
+      for (int i = lane * 2; i < D; i += 64) {
+        const float2 xv = __bfloat1622float2(*(const __nv_bfloat162*)(xr + i));
+        const float2 dv = __bfloat1622float2(*(const __nv_bfloat162*)(dr + i));
+        const float h0 = (xv.x - mu) * rs, h1 = (xv.y - mu) * rs;
+        float o0 = rs * (dv.x * g[i] - s1 - h0 * s2), o1 = rs * (dv.y * g[i + 1] - s1 - h1 * s2);
+        __nv_bfloat162* dst = (__nv_bfloat162*)(dx + (size_t)row * D + i);
+        if (dx_add) {
+          const float2 p = __bfloat1622float2(*dst);
+          o0 += p.x;
+          o1 += p.y;
+        }
+        *dst = __floats2bfloat162_rn(o0, o1);
+      }
     }
   }
   if (in_regs) {

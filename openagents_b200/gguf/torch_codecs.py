@@ -274,7 +274,7 @@ def repack_mxfp4(buf: torch.Tensor):
 
 def pack_mxfp4_wide(buf: torch.Tensor, rows: int):
     """Standard MXFP4 bytes of a matrix of ``rows`` rows -> (words [rows][K / 2] bytes, scales [ceil(K / 256)][rows][8]) as ``moe_qgemm.cu`` reads
-    them, or ``None`` where a block's scale is beyond what its arithmetic holds (2^1 and up; model weights are far below).
+    them, or ``None`` where a block's scale is beyond what its arithmetic holds (above 2^1; model weights are far below).
 
     Element i of a group of eight lies in half ``i % 2`` of a word; the half's four values at (sign bit, magnitude bits): (15, 8-6),
     (12, 5-3), (9, 2-0) and (13, 14 and 11-10).  A scale byte is the biased bf16 exponent of the block's scale times 2^126."""

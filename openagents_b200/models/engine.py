@@ -27,7 +27,7 @@ from ..utils.nvtx import nvtx_method
 
 MATVEC_MAX_TOKENS = 8
 QGEMM_MAX_TOKENS = 64      # tokens of a call up to which tensor-parallel ranks take the fused-dequant GEMM; also the row count of their slots
-FUSED_MAX_TOKENS = 384     # the same on one rank (see _layers_dense)
+FUSED_MAX_TOKENS = 3 * 128  # the same on one rank: three of that GEMM's token tiles (see _layers_dense)
 
 
 @dataclass
@@ -76,8 +76,8 @@ class LlamaEngine(PagedEngine):
         self._load(src)
         self._alloc()
         # Up to this many decode tokens take the mat-vec path, which multiplies by the weights as they are packed (whole numbers times 32-bit
-        # scales); the fused-dequant GEMM rounds them to bf16.  Measured on the 8B shape (ms per step, mat-vec / GEMM): 1 token
-        # 2.3 / 3.1, 2 tokens 2.9 / 3.1, 3 tokens 3.7 / 3.0, 8 tokens 5.0 / 3.0: at 3 and 4 the difference buys the weights' precision.
+        # scales); the fused-dequant GEMM rounds them to bf16.  Measured on the 8B shape (ms per step at 2048 tokens, mat-vec / GEMM): 1 token
+        # 2.25 / 2.76, 2 tokens 2.93 / 2.74, 4 tokens 3.74 / 2.86, 8 tokens 5.74 / 3.15: up to 4 the difference buys the weights' precision.
         self.small_path_tokens = min(MATVEC_MAX_TOKENS, int(os.environ.get("B200_SMALL_PATH_TOKENS", 4)))
         self.prefill_tc05 = os.environ.get("B200_PREFILL_TC05", "1") == "1"     # tcgen05 prefill attention (head sizes 64 and 128)
         self.seq_shard = os.environ.get("B200_TP_SEQ_SHARD", "1") == "1"        # sequence-sharded tensor-parallel prefill
@@ -350,8 +350,9 @@ class LlamaEngine(PagedEngine):
         """Any token count: tensor-core path.  Decode batches and short prompts run the projections whose weights are
         Q4_K / Q6_K on the fused-dequant GEMM, which streams the packed blocks, 128 tokens at a time; beyond
         FUSED_MAX_TOKENS every matrix is expanded into the shared scratch buffer and multiplied by the bf16 GEMM.
-        Measured on the 8B shape (ms per call, fused / expanded): 65 tokens 3.9 / 8.9, 128 tokens 4.0 / 8.2, 256
-        tokens 6.9 / 8.3, 384 tokens 10.2 / 10.2, 512 tokens 12.8 / 10.9."""
+        Its cost goes by tiles of 128 tokens, each of which expands all weights again; measured on the 8B shape (ms per call, fused /
+        expanded): 65 tokens 4.1 / 8.3, 128 tokens 4.2 / 8.3, 129 tokens 6.6 / 8.2, 256 tokens 7.1 / 8.3, 257 tokens 9.7 / 10.1, 300 tokens
+        9.9 / 10.3, 384 tokens 10.3 / 10.5, 400 tokens 12.8 / 10.4."""
         if self._seq_sharded(T, decode):
             return self._layers_seq_sharded(T, n_seqs, max_q)
         cfg, x = self.cfg, self.x[:T]
