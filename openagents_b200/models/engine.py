@@ -389,7 +389,7 @@ class LlamaEngine(PagedEngine):
                 if self._tc05_prefill(L, n_seqs, max_q, max_ctx_pages * PAGE):     # 5th-generation tensor-core path
                     ops.attn_prefill_tc05(self.q16, self.kc[li], self.vc[li], self.page_table, self.q_start, self.q_len,
                                           self.seq_lens, n_seqs, max_q, self.Hq, self.Hkv, window=L.window, sinks=L.sinks,
-                                          out_bf16=hb_q, status=self.status, dk=self.hd, dv=self.hd)
+                                          out_bf16=hb_q, status=self.status, dk=self.hd, dv=self.hd, exact_max=self.hd == 64)
                 else:
                     ops.attn_prefill(self.q16, self.kc[li], self.vc[li], self.page_table, self.max_pages, self.q_start,
                                      self.q_len, self.seq_lens, n_seqs, max_q, self.Hq, self.Hkv, self.hd, window=L.window,
@@ -469,7 +469,7 @@ class LlamaEngine(PagedEngine):
             if self._tc05_prefill(L, n_seqs, max_q, max_q):
                 ops.attn_prefill_tc05(self.q16, self.kc[li], self.vc[li], self.page_table, self.q_start, self.q_len,
                                       self.seq_lens, n_seqs, max_q, self.Hq, self.Hkv, window=L.window, sinks=L.sinks,
-                                      out_bf16=hb_q, status=self.status, dk=self.hd, dv=self.hd)
+                                      out_bf16=hb_q, status=self.status, dk=self.hd, dv=self.hd, exact_max=self.hd == 64)
             else:
                 ops.attn_prefill(self.q16, self.kc[li], self.vc[li], self.page_table, self.max_pages, self.q_start,
                                  self.q_len, self.seq_lens, n_seqs, max_q, self.Hq, self.Hkv, self.hd, window=L.window,

@@ -43,7 +43,7 @@ _SIGS = {
                          _P, _P, _P, _P, _P, _P],
     "b200_attn_prefill": [_P, _P, _P, _P, c_int, _P, _P, _P, _P, c_int, c_int, c_int, c_int, c_int, c_int, _P, _P, _P, _P],
     "b200_attn_prefill_tc05": [_P, _P, _P, _P, c_int, c_int, _P, _P, _P, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, _P, _P,
-                               c_int, _P, c_int, c_int, _P, _P, _P],
+                               c_int, _P, c_int, c_int, _P, c_int, _P, _P],
     "b200_attn_prefill_latent": [_P, _P, c_long, c_int, c_int, _P, _P, c_int, c_int, c_int, _P, c_int, _P, _P, _P] + [c_int] * 7 + [_P, _P, c_int, _P, _P, _P],
     "b200_gemm_bf16": [_P, _P, c_int, c_int, c_int, c_int, c_int, _P, _P, c_int, _P, _P, _P, c_int, c_int, c_int, c_int,
                        _P, c_int, _P, c_size_t, c_int, c_int, c_int, c_int, c_int, c_float, c_int, _P, c_int, _P],
@@ -281,12 +281,13 @@ def attn_prefill(q, kc, vc, page_table, max_pages, q_start, q_len, ctx_len, n_se
 
 
 def attn_prefill_tc05(q16, kc, vc, page_table, q_start, q_len, ctx_len, n_seqs, max_q_len, Hq, Hkv, window=0, sinks=None,
-                      out_bf16=None, status=None, dk=128, dv=128, gate=None, chunk=0, maps=1, out_f32=None):
+                      out_bf16=None, status=None, dk=128, dv=128, gate=None, chunk=0, maps=1, out_f32=None, exact_max=False):
     """``chunk`` > 0: keys of the query's own chunk only; ``maps`` 2: see :func:`qkv_finish`; ``out_f32`` instead of ``out_bf16``.  Prefill attention on tcgen05 (fp16 q / cache, bf16 out; ``dk`` 64..256 and ``dv`` 64 or 128, multiples of 64); ``gate``: fp32
-    [T, >= Hq] view whose sigmoid scales each head's output.  See ``attn_prefill_tc05.cu``."""
+    [T, >= Hq] view whose sigmoid scales each head's output; ``exact_max`` (head size 64): every row's weights relative to its own
+    maximum, as near to the exact result as :func:`attn_prefill`.  See ``attn_prefill_tc05.cu``."""
     _check(lib().b200_attn_prefill_tc05(_p(q16), _p(kc), _p(vc), _p(page_table), page_table.shape[1], kc.shape[0], _p(q_start),
                                         _p(q_len), _p(ctx_len), n_seqs, max_q_len, q16.shape[0], Hq, Hkv, dk, dv, window, _p(sinks),
-                                        _p(gate), 0 if gate is None else gate.stride(0), _p(out_bf16), chunk, maps, _p(out_f32), _p(status),
+                                        _p(gate), 0 if gate is None else gate.stride(0), _p(out_bf16), chunk, maps, _p(out_f32), int(exact_max), _p(status),
                                         _st()), "attn_prefill_tc05")
 
 

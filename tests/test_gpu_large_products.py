@@ -344,8 +344,9 @@ def test_routing_of_many_tokens(T, E, d, top_k):
         assert (recv[s.stop:(e + 1) * T] == 9.0).all()
 
 
+@pytest.mark.parametrize("exact", [False, True])
 @pytest.mark.parametrize("window,use_sinks", [(0, True), (1024, True), (1056, False), (0, False)])
-def test_prefill_attention_of_head_size_64(window, use_sinks):
+def test_prefill_attention_of_head_size_64(window, use_sinks, exact):
     """Head size 64 on tcgen05, with the long windows and sinks it takes there: cold prompts, chunks behind a context, one token, ends inside a block."""
     from test_gpu_kernels import _paged_kv
 
@@ -359,7 +360,7 @@ def test_prefill_attention_of_head_size_64(window, use_sinks):
     out, status = torch.zeros((sum(qlen), Hq * hd), dtype=torch.bfloat16, device=DEV), torch.zeros(1, dtype=torch.int32, device=DEV)
     i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)
     ops.attn_prefill_tc05(q, kc, vc, table, i32(starts), i32(qlen), i32(ctx), 4, max(qlen), Hq, Hkv, window=window, sinks=sinks, out_bf16=out,
-                          status=status, dk=hd, dv=hd)
+                          status=status, dk=hd, dv=hd, exact_max=exact)
     assert int(status) == 0
     for b in range(4):
         s, n = starts[b], qlen[b]
@@ -367,6 +368,27 @@ def test_prefill_attention_of_head_size_64(window, use_sinks):
                            window=window, sinks=None if sinks is None else sinks.cpu(), scale=1.0).reshape(n, -1)
         # probabilities in 16 bits (2^-11 of values of size about one, averaged) and the result in bf16
         assert ((out[s:s + n].float().cpu() - ref).abs() <= 2.0 ** -8 * ref.abs() + 4e-3).all(), b
+
+
+@pytest.mark.parametrize("gain", [0.3, 1.0, 3.0])                  # deviation of the scores: flat to peaked rows
+@pytest.mark.parametrize("T", [400, 1500])
+def test_prefill_attention_of_head_size_64_is_as_near_as_mma_sync(T, gain):
+    """The two kernels that serve head size 64, against 64 bits, on the same 16-bit inputs."""
+    from test_gpu_kernels import _paged_kv
+    ops, hd, Hq, Hkv = _ops(), 64, 8, 2
+    kc, vc, table, Ks, Vs = _paged_kv(1, Hkv, hd, [T], seed=91)
+    q = (_randn(T, Hq * hd, seed=92) * (gain / hd ** 0.5)).half()
+    i32 = lambda v: torch.tensor([v], dtype=torch.int32, device=DEV)
+    a, b, status = torch.empty((T, Hq * hd), device=DEV), torch.empty((T, Hq * hd), device=DEV), torch.zeros(1, dtype=torch.int32, device=DEV)
+    ops.attn_prefill_tc05(q, kc, vc, table, i32(0), i32(T), i32(T), 1, T, Hq, Hkv, out_f32=a, status=status, dk=hd, dv=hd, exact_max=True)
+    ops.attn_prefill(q, kc, vc, table, table.shape[1], i32(0), i32(T), i32(T), 1, T, Hq, Hkv, hd, out_f32=b)
+    K, V = (t[0].double().to(DEV).repeat_interleave(Hq // Hkv, 1) for t in (Ks, Vs))
+    s = torch.einsum("thd,shd->hts", q.double().view(T, Hq, hd), K).masked_fill(torch.ones(T, T, device=DEV).triu(1).bool(), float("-inf"))
+    ref = torch.einsum("hts,shd->thd", s.softmax(-1), V).reshape(T, -1)
+    # norms of T * 512 errors scatter by far less than 2 %
+    assert (a - ref).norm() <= 1.02 * (b - ref).norm() and int(status) == 0
+    with pytest.raises(RuntimeError):
+        ops.attn_prefill_tc05(q.view(-1, 128).repeat(1, 8), kc, vc, table, i32(0), i32(T), i32(T), 1, T, Hq, Hkv, out_f32=a, exact_max=True)
 
 
 # K of one K block, of a two-block stage and a half, of a ring that just fits, wraps, and wraps with a remainder; columns for tiles of 64, 128 and 256
